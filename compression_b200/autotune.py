@@ -3,12 +3,9 @@
 Every knob of include/gd.h (gd_tune_key) selects among kernel variants that
 are compiled into libgd.so or sets a launch shape:
 
-  inflate  GD_TUNE_INFLATE_VARIANT        1, 2: one warp per stream, no window, 2 / 4 per block
-                                          3: one warp per stream with a 32 KiB window
-                                          4, 5: decoder + writer pair, no window, 2 / 4 per block
-                                          6: decoder + writer pair with the window
-                                          7-13: pairs with a 16 / 8 / 4 KiB window, smaller buffers
-                                          0: 12 for >= 4 streams per SM, else 6
+  inflate  GD_TUNE_INFLATE_VARIANT        1-4: a block per stream, one, two, three or four blocks per SM
+                                          6, 12: decoder + writer warp pair, a 32 / 4 KiB window
+                                          0: 1, 2 or 3 by the number of streams
   brle     GD_TUNE_BRLE_BLOCKS_PER_SM     grid = value x SMs
   rlev1    GD_TUNE_RLEV1_LANES_PER_BLOCK  lane streams (warps) per block
   rlev2    GD_TUNE_RLEV2_LANES_PER_BLOCK  lane streams (warps) per block
@@ -48,7 +45,7 @@ TUNE_LZSS_WARPS_PER_BLOCK = 4
 
 # codec -> (knob, candidate values; the first is the built-in default)
 KNOBS = {
-    "deflate": (TUNE_INFLATE_VARIANT, [0, 6, 12, 10, 4]),
+    "deflate": (TUNE_INFLATE_VARIANT, [0, 1, 2, 3, 4]),
     "brle": (TUNE_BRLE_BLOCKS_PER_SM, [8, 4, 16]),
     "rlev1": (TUNE_RLEV1_LANES_PER_BLOCK, [8, 4]),
     "rlev2": (TUNE_RLEV2_LANES_PER_BLOCK, [8, 4]),

@@ -1,7 +1,8 @@
-// inflate.cu -- Deflate / zlib inflate kernels for sm_100a: one warp per
-// stream (the warp-level decoder is in inflate.cuh), with offset-array and
-// cuDF-descriptor front ends.
+// inflate.cu -- Deflate / zlib inflate kernels for sm_100a: a block per stream
+// (inflate_block.cuh) or, by knob, a warp pair per stream (inflate.cuh), with
+// offset-array and cuDF-descriptor front ends.
 #include "inflate.cuh"
+#include "inflate_block.cuh"
 
 namespace gd {
 namespace infl {
@@ -43,29 +44,6 @@ struct CudfChunks {
         st[c].reserved = 0;
     }
 };
-
-// NW warps per block, one stream per warp; WIN: output window (see
-// WarpSmemT).  Blocks are handed out by the hardware in launch order, so
-// `order` (longest first, say) is also the order streams start in.
-template <class Chunks, uint32_t WIN, int NW>
-__global__ void __launch_bounds__(NW * 32) inflate_kernel(Chunks ch, uint32_t n_chunks, int zlib_hdr,
-                                                         const uint32_t* __restrict__ order) {
-    extern __shared__ __align__(16) uint8_t smem_raw[];
-    const uint32_t wid = threadIdx.x >> 5;
-    const uint32_t slot = blockIdx.x * NW + wid;
-    if (slot >= n_chunks) return;
-    const uint32_t chunk = order ? order[slot] : slot;
-    WarpSmemT<WIN>& S = *reinterpret_cast<WarpSmemT<WIN>*>(smem_raw + wid * sizeof(WarpSmemT<WIN>));
-    const uint8_t* src;
-    uint8_t* dst;
-    uint64_t clen64, olen64;
-    uint32_t err = ch.get(chunk, src, clen64, dst, olen64) ? ST_OK : ST_CORRUPT;
-    if (olen64 > 0xffffffffull || clen64 > 0xffffffffull) err = ST_CORRUPT;
-    uint32_t fin = 0;
-    if (err == ST_OK) err = stream_warp_impl<WIN>(src, (uint32_t)clen64, dst, (uint32_t)olen64, zlib_hdr, S, &fin);
-    if (err == ST_OK && Chunks::exact && fin != (uint32_t)olen64) err = ST_CORRUPT;
-    if (lane_id() == 0) ch.put(chunk, err, err == ST_OK ? fin : 0);
-}
 
 // Reader/writer pairs: NP pairs per block, warps 2i (decoder) and 2i+1
 // (writer) share stream i's state and hand batches over through it.
@@ -110,6 +88,29 @@ __global__ void __launch_bounds__(NP * 64) inflate_pair_kernel(Chunks ch, uint32
 }
 
 }  // namespace infl
+
+namespace inflb {
+
+// A block per stream.  Blocks are handed out by the hardware in launch order,
+// so `order` (longest first, say) is also the order streams start in.
+template <class Chunks, class SmemT, int BPS>
+__global__ void __launch_bounds__(SmemT::NT, BPS) inflate_block_kernel(Chunks ch, int zlib_hdr,
+                                                                 const uint32_t* __restrict__ order) {
+    extern __shared__ __align__(16) uint8_t smem_raw[];
+    SmemT& S = *reinterpret_cast<SmemT*>(smem_raw);
+    const uint32_t chunk = order ? order[blockIdx.x] : blockIdx.x;
+    const uint8_t* src;
+    uint8_t* dst;
+    uint64_t clen64, olen64;
+    uint32_t err = ch.get(chunk, src, clen64, dst, olen64) ? ST_OK : ST_CORRUPT;
+    if (olen64 > 0xffffffffull || clen64 > 0xffffffffull) err = ST_CORRUPT;
+    uint32_t fin = 0;
+    if (err == ST_OK) err = stream_block(src, (uint32_t)clen64, dst, (uint32_t)olen64, zlib_hdr, S, &fin);
+    if (err == ST_OK && Chunks::exact && fin != (uint32_t)olen64) err = ST_CORRUPT;
+    if (threadIdx.x == 0) ch.put(chunk, err, err == ST_OK ? fin : 0);
+}
+
+}  // namespace inflb
 }  // namespace gd
 
 namespace {
@@ -120,22 +121,6 @@ __global__ void copy_uncompressed_kernel(const gd_inflate_input* in, int count) 
     uint8_t* d = static_cast<uint8_t*>(in[c].dstDevice);
     const uint64_t n = min(in[c].srcSize, in[c].dstSize);
     for (uint64_t i = threadIdx.x; i < n; i += blockDim.x) d[i] = s[i];
-}
-
-template <class Chunks, uint32_t WIN, int NW>
-gd_status_t launch_cfg(const Chunks& ch, uint32_t n, int zlib_hdr, const uint32_t* order, cudaStream_t s) {
-    using namespace gd::infl;
-    const uint32_t smem = NW * (uint32_t)sizeof(WarpSmemT<WIN>);
-    static bool attr_set = false;  // benign race: the attribute call is idempotent
-    if (!attr_set) {
-        if (cudaFuncSetAttribute(inflate_kernel<Chunks, WIN, NW>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 smem) != cudaSuccess)
-            return GD_ERR_CUDA;
-        attr_set = true;
-    }
-    const uint32_t grid = (n + NW - 1) / NW;
-    inflate_kernel<Chunks, WIN, NW><<<grid, NW * 32, smem, s>>>(ch, n, zlib_hdr, order);
-    return cudaGetLastError() == cudaSuccess ? GD_OK : GD_ERR_CUDA;
 }
 
 template <class Chunks, uint32_t WIN, int NP, uint32_t RB = gd::infl::IRING, uint32_t DB = gd::infl::LBITS,
@@ -158,40 +143,46 @@ gd_status_t launch_pair(const Chunks& ch, uint32_t n, int zlib_hdr, const uint32
     return cudaGetLastError() == cudaSuccess ? GD_OK : GD_ERR_CUDA;
 }
 
-// Launch configuration (GD_TUNE_INFLATE_VARIANT): 1 / 2 = one warp per
-// stream without a window, 2 / 4 warps per block; 3 = one warp per stream
-// with a window; 4 / 5 = decoder/writer warp pairs without a window (copies
-// read the output), 2 / 4 pairs per block; 6 = one decoder/writer pair per
-// block with a 32 KiB shared window; 7 - 13 = pairs with a 16 / 8 / 4 KiB
-// window (nearer copies from shared memory, farther ones from the output)
-// and smaller rings, distance tables and batches, so that 7 to 15 pairs fit
-// on an SM; 0 (default) = 12 for at least 4 streams per SM, else 6.
+template <int NW, uint32_t WIN, uint32_t NC, uint32_t TMAX, int BPS, class Chunks>
+gd_status_t launch_block(const Chunks& ch, uint32_t n, int zlib_hdr, const uint32_t* order, cudaStream_t s) {
+    using SmemT = gd::inflb::Smem<NW, WIN, NC, TMAX>;
+    auto kern = gd::inflb::inflate_block_kernel<Chunks, SmemT, BPS>;
+    static bool attr_set = false;  // benign race: the attribute call is idempotent
+    if (!attr_set) {
+        if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, sizeof(SmemT)) != cudaSuccess)
+            return GD_ERR_CUDA;
+        attr_set = true;
+    }
+    kern<<<n, SmemT::NT, sizeof(SmemT), s>>>(ch, zlib_hdr, order);
+    return cudaGetLastError() == cudaSuccess ? GD_OK : GD_ERR_CUDA;
+}
+
+// Launch configuration (GD_TUNE_INFLATE_VARIANT): 1 - 4 = a block per stream;
+// 6 / 12 = a decoder warp (one lane at work) and a writer warp per stream with
+// a 32 / 4 KiB window, whose hand-off wait the test knobs bound; any other
+// value = by the number of streams:
+//   up to one a SM: 16 warps and the largest window and placement (39 streams
+//   of 128 KiB: 0.107 ms; 8 warps 0.165; the warp pair 1.05);
+//   up to two a SM: 8 warps, two blocks a SM;
+//   more: 8 warps, three blocks a SM (2048 streams of 4 KiB to 700 KiB,
+//   256 MiB: 1.04 ms; two blocks with twice the placement 1.10; 4 warps
+//   1.47; 16 warps 1.16; the warp pair 5.09).
 template <class Chunks>
 gd_status_t launch_inflate(const Chunks& ch, uint32_t n, int zlib_hdr, const uint32_t* order, cudaStream_t s) {
     int v = gd_tune_get(GD_TUNE_INFLATE_VARIANT);
-    if (v == 0) {
-        // many streams: throughput, i.e. more pairs per SM (no window); few:
-        // the fastest single stream (window)
+    if (v < 1 || (v > 4 && v != 6 && v != 12)) {
         int dev = 0, sms = 148;
         cudaGetDevice(&dev);
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-        v = n >= 4u * (uint32_t)sms ? 12 : 6;
+        v = n <= (uint32_t)sms ? 1 : n <= 2u * (uint32_t)sms ? 2 : 3;
     }
     switch (v) {
-        case 1: return launch_cfg<Chunks, 0, 2>(ch, n, zlib_hdr, order, s);
-        case 2: return launch_cfg<Chunks, 0, 4>(ch, n, zlib_hdr, order, s);
-        case 3: return launch_cfg<Chunks, 32768, 1>(ch, n, zlib_hdr, order, s);
-        case 4: return launch_pair<Chunks, 0, 2>(ch, n, zlib_hdr, order, s);
-        case 5: return launch_pair<Chunks, 0, 4>(ch, n, zlib_hdr, order, s);
-        case 7: return launch_pair<Chunks, 16384, 1, 2048, 8, 1024, 128>(ch, n, zlib_hdr, order, s);
-        case 8: return launch_pair<Chunks, 16384, 2, 2048, 8, 1024, 128>(ch, n, zlib_hdr, order, s);
-        case 9: return launch_pair<Chunks, 8192, 1, 2048, 8, 1024, 128>(ch, n, zlib_hdr, order, s);
-        case 10: return launch_pair<Chunks, 4096, 1, 2048, 8, 1024, 128>(ch, n, zlib_hdr, order, s);
-        case 11: return launch_pair<Chunks, 8192, 1, 1024, 8, 512, 64>(ch, n, zlib_hdr, order, s);
+        case 1: return launch_block<16, 65536, 8192, 32608, 1>(ch, n, zlib_hdr, order, s);
+        case 2: return launch_block<8, 32768, 4096, 16224, 2>(ch, n, zlib_hdr, order, s);
+        case 4: return launch_block<8, 16384, 2048, 8032, 4>(ch, n, zlib_hdr, order, s);
+        case 6: return launch_pair<Chunks, 32768, 1>(ch, n, zlib_hdr, order, s);
         case 12: return launch_pair<Chunks, 4096, 1, 1024, 8, 512, 64>(ch, n, zlib_hdr, order, s);
-        case 13: return launch_pair<Chunks, 4096, 2, 1024, 8, 512, 64>(ch, n, zlib_hdr, order, s);
-        case 14: return launch_pair<Chunks, 2048, 1, 1024, 8, 512, 64>(ch, n, zlib_hdr, order, s);
-        default: return launch_pair<Chunks, 32768, 1>(ch, n, zlib_hdr, order, s);
+        default: return launch_block<8, 32768, 2048, 8032, 3>(ch, n, zlib_hdr, order, s);
     }
 }
 }  // namespace

@@ -284,17 +284,12 @@ gd_status_t gd_batch_decode_lpt_noalloc(const gd_task* d_tasks, uint32_t n_tasks
  * autotuner, which times the choices on the device.
  * ------------------------------------------------------------------------ */
 typedef enum gd_tune_key {
-    GD_TUNE_INFLATE_VARIANT = 0, /* 1 / 2: one warp per stream, no window, 2 / 4 warps per block;
-                                    3: one warp per stream with a 32 KiB shared output window;
-                                    4 / 5: decoder + writer warp pair per stream, no window
-                                    (copies read the output), 2 / 4 pairs per block;
-                                    6: decoder + writer pair with the window, one per block;
-                                    7 / 8: pairs with a 16 KiB window, 1 / 2 per block;
-                                    9 / 10: 8 / 4 KiB window; 11 / 12: 8 / 4 KiB window with a
-                                    1 KiB ring and batches of 512 literals / 64 commands;
-                                    13: as 12, 2 pairs per block (copies beyond the window
-                                    read the output); 14: as 12 with a 2 KiB window;
-                                    0 (default): 12 for >= 4 streams per SM, else 6 */
+    GD_TUNE_INFLATE_VARIANT = 0, /* 1 - 4: a block per stream: 16 warps and a 64 KiB output window, one
+                                    block per SM; 8 warps and a 32 KiB window, two; the same with
+                                    smaller steps, three; 8 warps and a 16 KiB window, four;
+                                    6 / 12: decoder + writer warp pair per stream, a 32 / 4 KiB window;
+                                    any other value (0, the default): 1 for up to one stream per SM,
+                                    2 for up to two, else 3 */
     GD_TUNE_BRLE_BLOCKS_PER_SM = 1,   /* byte-RLE grid = value x SMs blocks (default 8) */
     GD_TUNE_RLEV1_LANES_PER_BLOCK = 2, /* 0/8: 8 lane streams per block; 4: 4 */
     GD_TUNE_RLEV2_LANES_PER_BLOCK = 3, /* 0: 8 lane streams per block (4 if 8 do not fit in shared
