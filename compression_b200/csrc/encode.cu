@@ -5,25 +5,24 @@
 // rlev2::compress_gpu_transpose, include/rlev2/encoder_trans.h:428-537),
 // producing the same bytes as the host encoders (both run the lane encoders
 // of lane_enc.h).  Three launches on one stream:
-//   1. lane_encode_kernel: a warp per chunk, a thread per lane stream.  Each
-//      thread gathers its lane's values straight from the column (RLE v1:
-//      COMP_COL_LEN-byte slices at a 32-slice stride; RLE v2: READ_UNIT-value
-//      slices) and runs the lane encoder into its own scratch slot, buffering
-//      4 bytes in a register so the scratch is written in whole words (the
-//      literal-count byte written back later is a byte store or a register
-//      edit).  The warp sums its lanes' padded word counts into the chunk's
-//      block size;
+//   1. the lane streams: RLE v1, lane_encode_kernel: a warp per chunk, a
+//      thread per lane stream.  Each thread gathers its lane's values straight
+//      from the column (COMP_COL_LEN-byte slices at a 32-slice stride) and runs
+//      the lane encoder into its own scratch slot, buffering 4 bytes in a
+//      register so the scratch is written in whole words (the literal-count
+//      byte written back later is a byte store or a register edit).  RLE v2: a
+//      warp per lane stream (rlev2_enc.cuh), then a warp per chunk sums the
+//      padded word counts into the block size (lane_encode_kernel does that
+//      itself);
 //   2. offsets_kernel: one block turns the block sizes into blk_off;
-//   3. interleave_kernel: a block per chunk writes row k = one word of every
-//      lane longer than 4k bytes, in lane order, through the same segment
-//      table the decoders read with (interleave.cuh), then zeroes the block's
-//      pad to 128 bytes.
-// The encoders are serial per lane, so the first launch has one thread per
-// lane stream (32 x chunks); the column is read once and the scratch and the
-// container written once each.
+//   3. interleave_kernel: row k = one word of every lane longer than 4k bytes,
+//      in lane order, through the same segment table the decoders read with
+//      (interleave.cuh), then the block's pad to 128 bytes zeroed.
+// The column is read once and the scratch and the container written once each.
 #include "gd_common.cuh"
 #include "interleave.cuh"
 #include "lane_enc.h"
+#include "rlev2_enc.cuh"
 
 namespace gd {
 namespace encd {
@@ -71,25 +70,10 @@ struct V1Vals {
     }
 };
 
-// RLE v2 lane t: value i is chunk value t * ru + (i / ru) * 32 * ru + i % ru
-// (encoder_trans.h:40-108); values past the input are zero.
-struct V2Vals {
-    const int64_t* base;
-    uint64_t avail;
-    uint32_t t, ru;
-    __device__ __forceinline__ int64_t operator[](uint64_t i) const {
-        const uint32_t q = (uint32_t)i / ru, r = (uint32_t)i - q * ru;
-        const uint64_t idx = (uint64_t)t * ru + (uint64_t)q * 32u * ru + r;
-        return idx < avail ? base[idx] : 0;
-    }
-};
-
-// CODEC: GD_CODEC_RLEV1 (T = uint32_t / uint64_t, param = wil) or
-// GD_CODEC_RLEV2 (T = int64_t, param = read unit).  blk_size[c] gets chunk
-// c's block size (the launch passes blk_off + 1).
-template <int CODEC, typename T>
+// RLE v1: blk_size[c] gets chunk c's block size (the launch passes blk_off + 1).
+template <typename T>
 __global__ void __launch_bounds__(NT) lane_encode_kernel(const uint8_t* __restrict__ in, uint64_t n_bytes,
-                                                         uint32_t n_chunks, uint64_t chunk_size, uint32_t param,
+                                                         uint32_t n_chunks, uint64_t chunk_size, uint32_t wil,
                                                          uint8_t* __restrict__ scratch, uint32_t lane_cap,
                                                          uint64_t* __restrict__ col_len,
                                                          uint64_t* __restrict__ blk_size,
@@ -100,13 +84,8 @@ __global__ void __launch_bounds__(NT) lane_encode_kernel(const uint8_t* __restri
     const uint64_t cb = (uint64_t)c * chunk_size;
     const uint64_t have = n_bytes > cb ? (n_bytes - cb < chunk_size ? n_bytes - cb : chunk_size) : 0;
     DevSink s{reinterpret_cast<uint32_t*>(scratch + ((uint64_t)c * 32u + t) * lane_cap), 0u, lane_cap, 0u};
-    if constexpr (CODEC == GD_CODEC_RLEV1) {
-        const V1Vals<T> v{reinterpret_cast<const T*>(in + cb), have / sizeof(T), t, param};
-        enc::rlev1_encode_lane<T>(v, chunk_size / 32u / sizeof(T), s);
-    } else {
-        const V2Vals v{reinterpret_cast<const int64_t*>(in + cb), have / 8u, t, param};
-        enc::rlev2_encode_lane(v, chunk_size / 256u, s);
-    }
+    const V1Vals<T> v{reinterpret_cast<const T*>(in + cb), have / sizeof(T), t, wil};
+    enc::rlev1_encode_lane<T>(v, chunk_size / 32u / sizeof(T), s);
     s.flush();
     const bool over = s.n > lane_cap;
     const uint32_t len = over ? 0u : s.n;
@@ -137,9 +116,13 @@ __global__ void __launch_bounds__(1024) offsets_kernel(uint64_t* __restrict__ bl
     if (threadIdx.x == 0) blk_off[0] = 0;
 }
 
-// Block c = slots' words in rows; a block of NT threads per chunk.  Slot t's
-// stream is scratch slot col_map[32c + t] of the chunk (LZSS: slots are
-// length ranks) or slot t (col_map null).
+// Block c = slots' words in rows.  Slot t's stream is scratch slot
+// col_map[32c + t] of the chunk (LZSS: slots are length ranks) or slot t
+// (col_map null).  A block takes the chunk's tiles of 32 rows, every gridDim.y-th
+// one: the 32 slots' words are read 128 bytes at a time, turned in shared
+// memory, and every row is written by a warp, its words side by side.  (A warp
+// per slot, storing one word in every row, wrote a sector per word: 0.124
+// against 0.034 ms for 47 MB of RLE v1 streams.)
 __global__ void __launch_bounds__(NT) interleave_kernel(const uint8_t* __restrict__ scratch, uint32_t lane_cap,
                                                         const uint64_t* __restrict__ col_len,
                                                         const uint64_t* __restrict__ blk_off, uint32_t n_chunks,
@@ -148,12 +131,15 @@ __global__ void __launch_bounds__(NT) interleave_kernel(const uint8_t* __restric
     __shared__ SegTable T;
     __shared__ uint32_t s_nw[32];
     __shared__ uint32_t s_tot;
+    __shared__ uint32_t s_slot[32];
+    __shared__ uint32_t s_tile[32][33];
     const uint32_t lane = lane_id(), wid = threadIdx.x >> 5;
     for (uint32_t c = blockIdx.x; c < n_chunks; c += gridDim.x) {
         if (wid == 0) {
             const uint32_t nw = (uint32_t)((col_len[(uint64_t)c * 32u + lane] + 3u) >> 2);
             seg_build(&T, nw);
             s_nw[lane] = nw;
+            s_slot[lane] = col_map ? (col_map[(uint64_t)c * 32u + lane] & 31u) : lane;
             const uint32_t tot = __reduce_add_sync(GD_FULL_MASK, nw);
             if (lane == 0) s_tot = tot;
         }
@@ -161,24 +147,40 @@ __global__ void __launch_bounds__(NT) interleave_kernel(const uint8_t* __restric
         const uint64_t b0 = blk_off[c];
         uint32_t* dst = reinterpret_cast<uint32_t*>(data + b0);
         const uint32_t* src0 = reinterpret_cast<const uint32_t*>(scratch + (uint64_t)c * 32u * lane_cap);
-        for (uint32_t t = wid; t < 32; t += NT / 32) {
-            const uint32_t nw = s_nw[t], ltmask = (1u << t) - 1u;
-            const uint32_t st = col_map ? (col_map[(uint64_t)c * 32u + t] & 31u) : t;
-            const uint32_t* src = src0 + (uint64_t)st * (lane_cap / 4u);
-            for (uint32_t k = lane; k < nw; k += 32) {
-                uint32_t j = 0;  // segment of row k: the number of lanes with at most k words
+        const uint32_t nw = s_nw[lane], rows = T.hi[31];
+        for (uint32_t k0 = 32u * blockIdx.y; k0 < rows; k0 += 32u * gridDim.y) {
 #pragma unroll
-                for (uint32_t step = 16; step; step >>= 1)
-                    if (j + step <= 31 && T.hi[j + step - 1] <= k) j += step;
-                const uint32_t lo = j ? T.hi[j - 1] : 0u;
-                const uint32_t off = T.base[j] + (k - lo) * 4u * (32u - j) + 4u * __popc(T.mask[j] & ltmask);
-                dst[off >> 2] = src[k];
+            for (uint32_t t = wid; t < 32; t += NT / 32)
+                s_tile[t][lane] = k0 + lane < s_nw[t] ? src0[(uint64_t)s_slot[t] * (lane_cap / 4u) + k0 + lane] : 0u;
+            __syncthreads();
+#pragma unroll
+            for (uint32_t r = wid; r < 32; r += NT / 32) {
+                const uint32_t k = k0 + r;
+                const uint32_t act = __ballot_sync(GD_FULL_MASK, nw > k), j = 32u - __popc(act);
+                if (nw > k) {
+                    const uint32_t lo = j ? T.hi[j - 1] : 0u;
+                    const uint32_t off = (T.base[j] >> 2) + (k - lo) * (32u - j);
+                    dst[off + __popc(act & ((1u << lane) - 1u))] = s_tile[lane][r];
+                }
             }
+            __syncthreads();
         }
         const uint32_t bw = (uint32_t)((blk_off[c + 1] - b0) >> 2);
-        for (uint32_t w = s_tot + threadIdx.x; w < bw; w += NT) dst[w] = 0;
+        if (blockIdx.y == 0)
+            for (uint32_t w = s_tot + threadIdx.x; w < bw; w += NT) dst[w] = 0;
         __syncthreads();  // T and s_nw are rebuilt for the next chunk
     }
+}
+
+// Grid of interleave_kernel: blocks for every chunk, and for every four tiles
+// of the longest stream a slot can hold, up to 8 a chunk.
+inline dim3 interleave_grid(uint64_t n_chunks, uint64_t lane_cap) {
+    int dev = 0, sms = 148;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    const uint64_t x = n_chunks < (uint64_t)sms * 16u ? n_chunks : (uint64_t)sms * 16u;
+    const uint64_t y = lane_cap / 512u;
+    return dim3((uint32_t)x, (uint32_t)(y < 1 ? 1 : y > 8 ? 8 : y));
 }
 
 // ---------------------------------------------------------------------------
@@ -401,21 +403,12 @@ inline uint64_t rlev2_lane_cap(uint64_t chunk_size) {
     return (nv * 11u + 64u + 3u) & ~3ull;
 }
 
-template <typename Kern>
-gd_status_t run(Kern k1, const uint8_t* d_in, uint64_t n_bytes, uint64_t chunk_size, uint32_t param,
-                uint64_t lane_cap, uint8_t* d_scratch, uint8_t* d_data, uint64_t* d_blk_off, uint64_t* d_col_len,
-                uint32_t* d_status, cudaStream_t s) {
-    const uint64_t nc = (n_bytes + chunk_size - 1) / chunk_size;
-    const uint32_t grid1 = (uint32_t)((nc + NT / 32 - 1) / (NT / 32));
-    k1<<<grid1, NT, 0, s>>>(d_in, n_bytes, (uint32_t)nc, chunk_size, param, d_scratch, (uint32_t)lane_cap,
-                            d_col_len, d_blk_off + 1, d_status);
+// blk_off from the block sizes, then the container.
+inline gd_status_t finish(uint64_t nc, const uint8_t* d_scratch, uint64_t lane_cap, uint8_t* d_data,
+                          uint64_t* d_blk_off, const uint64_t* d_col_len, const uint8_t* d_col_map, cudaStream_t s) {
     offsets_kernel<<<1, 1024, 0, s>>>(d_blk_off, (uint32_t)nc);
-    int dev = 0, sms = 148;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    const uint64_t g3 = nc < (uint64_t)sms * 16u ? nc : (uint64_t)sms * 16u;
-    interleave_kernel<<<(uint32_t)g3, NT, 0, s>>>(d_scratch, (uint32_t)lane_cap, d_col_len, d_blk_off,
-                                                  (uint32_t)nc, d_data);
+    interleave_kernel<<<interleave_grid(nc, lane_cap), NT, 0, s>>>(d_scratch, (uint32_t)lane_cap, d_col_len, d_blk_off,
+                                                                  (uint32_t)nc, d_data, d_col_map);
     return cudaGetLastError() == cudaSuccess ? GD_OK : GD_ERR_CUDA;
 }
 
@@ -448,11 +441,12 @@ extern "C" gd_status_t gd_rlev1_encode_device(const uint8_t* d_in, uint64_t n_by
     const uint64_t cap = rlev1_lane_cap(chunk_size, elem_bytes);
     const uint32_t wil = comp_col_len / elem_bytes;
     cudaStream_t s = (cudaStream_t)stream;
-    if (elem_bytes == 4)
-        return run(lane_encode_kernel<GD_CODEC_RLEV1, uint32_t>, d_in, n_bytes, chunk_size, wil, cap, d_scratch,
-                   d_data, d_blk_off, d_col_len, d_status, s);
-    return run(lane_encode_kernel<GD_CODEC_RLEV1, uint64_t>, d_in, n_bytes, chunk_size, wil, cap, d_scratch, d_data,
-               d_blk_off, d_col_len, d_status, s);
+    const uint64_t nc = (n_bytes + chunk_size - 1) / chunk_size;
+    auto kern = elem_bytes == 4 ? lane_encode_kernel<uint32_t> : lane_encode_kernel<uint64_t>;
+    kern<<<(uint32_t)((nc + NT / 32 - 1) / (NT / 32)), NT, 0, s>>>(d_in, n_bytes, (uint32_t)nc, chunk_size, wil,
+                                                                   d_scratch, (uint32_t)cap, d_col_len, d_blk_off + 1,
+                                                                   d_status);
+    return finish(nc, d_scratch, cap, d_data, d_blk_off, d_col_len, nullptr, s);
 }
 
 extern "C" uint64_t gd_rlev2_encode_bound(uint64_t n_bytes, uint64_t chunk_size) {
@@ -472,8 +466,12 @@ extern "C" gd_status_t gd_rlev2_encode_device(const uint8_t* d_in, uint64_t n_by
         (reinterpret_cast<uintptr_t>(d_data) & 3u))
         return GD_ERR_INVALID_ARG;
     if ((n_bytes + chunk_size - 1) / chunk_size > 0xffffffffull) return GD_ERR_UNSUPPORTED;
-    return run(lane_encode_kernel<GD_CODEC_RLEV2, int64_t>, d_in, n_bytes, chunk_size, read_unit,
-               rlev2_lane_cap(chunk_size), d_scratch, d_data, d_blk_off, d_col_len, d_status, (cudaStream_t)stream);
+    const uint64_t nc = (n_bytes + chunk_size - 1) / chunk_size, cap = rlev2_lane_cap(chunk_size);
+    cudaStream_t s = (cudaStream_t)stream;
+    rlev2_encode_kernel<<<(uint32_t)((nc * 32u + V2_WPB - 1) / V2_WPB), V2_WPB * 32, 0, s>>>(
+        d_in, n_bytes, nc * 32u, chunk_size, read_unit, d_scratch, (uint32_t)cap, d_col_len);
+    lane_sizes_kernel<<<(uint32_t)((nc + 3) / 4), 128, 0, s>>>((uint32_t)nc, d_col_len, d_blk_off + 1, d_status);
+    return finish(nc, d_scratch, cap, d_data, d_blk_off, d_col_len, nullptr, s);
 }
 
 extern "C" uint64_t gd_lzss_encode_bound(uint64_t n_bytes, uint64_t chunk_size) {
@@ -504,14 +502,7 @@ extern "C" gd_status_t gd_lzss_encode_device(const uint8_t* d_in, uint64_t n_byt
         d_in, n_bytes, chunk_size, ncol, d_scratch, (uint32_t)cap, raw_len, wsm);
     lzss_rank_kernel<<<(uint32_t)((nc + NT / 32 - 1) / (NT / 32)), NT, 0, s>>>(raw_len, (uint32_t)nc, d_col_len,
                                                                               d_col_map, d_blk_off + 1, d_status);
-    offsets_kernel<<<1, 1024, 0, s>>>(d_blk_off, (uint32_t)nc);
-    int dev = 0, sms = 148;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    const uint64_t g3 = nc < (uint64_t)sms * 16u ? nc : (uint64_t)sms * 16u;
-    interleave_kernel<<<(uint32_t)g3, NT, 0, s>>>(d_scratch, (uint32_t)cap, d_col_len, d_blk_off, (uint32_t)nc, d_data,
-                                                  d_col_map);
-    return cudaGetLastError() == cudaSuccess ? GD_OK : GD_ERR_CUDA;
+    return finish(nc, d_scratch, cap, d_data, d_blk_off, d_col_len, d_col_map, s);
 }
 
 // ---------------------------------------------------------------------------
@@ -632,12 +623,5 @@ extern "C" gd_status_t gd_brle_trans_encode_device(const uint8_t* d_in, uint64_t
                                                                  (uint32_t)cap, raw_len);
     lzss_rank_kernel<<<(uint32_t)((nc + NT / 32 - 1) / (NT / 32)), NT, 0, s>>>(raw_len, (uint32_t)nc, d_col_len,
                                                                               d_col_map, d_blk_off + 1, d_status);
-    offsets_kernel<<<1, 1024, 0, s>>>(d_blk_off, (uint32_t)nc);
-    int dev = 0, sms = 148;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    const uint64_t g3 = nc < (uint64_t)sms * 16u ? nc : (uint64_t)sms * 16u;
-    interleave_kernel<<<(uint32_t)g3, NT, 0, s>>>(d_scratch, (uint32_t)cap, d_col_len, d_blk_off, (uint32_t)nc, d_data,
-                                                  d_col_map);
-    return cudaGetLastError() == cudaSuccess ? GD_OK : GD_ERR_CUDA;
+    return finish(nc, d_scratch, cap, d_data, d_blk_off, d_col_len, d_col_map, s);
 }
