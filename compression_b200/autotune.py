@@ -14,7 +14,7 @@ are compiled into libgd.so or sets a launch shape:
                                           16 / 8 lanes per column, 1: a lane per column (these stage
                                           the whole chunk in shared memory)
 
-For the batched decoder the tuned quantity is its blocks per SM (4 warps each),
+For the batched decoder the tuned quantity is its blocks per SM (8 warps each),
 which sets how many tasks run at once against how much shared memory each
 gets.
 

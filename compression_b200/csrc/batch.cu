@@ -1,17 +1,28 @@
 // batch.cu -- batched mixed-codec decoding: one persistent launch over a
-// list of warp-sized tasks of any codec, fed from a device work queue.
+// list of tasks of any codec, fed from a device work queue.
 //
 // No counterpart in the reference (its decoders are one launch per column
 // and codec).  A task is one brle chunk, one RLE v1 / RLE v2 lane stream,
-// one LZSS chunk or one Deflate stream; every codec has a warp-level decoder
-// (brle_warp.cuh, rlev1.cuh, rlev2.cuh, lzss.cuh, inflate.cuh), so a single
-// kernel can run them all.  Each warp repeatedly takes the next task either
-// from a global atomic counter over an order array (dynamic: with tasks
-// sorted longest-first this is LPT list scheduling) or by the static mapping
-// task i -> warp i mod W.  Per-task %globaltimer start/end stamps (optional)
-// are the measurements the learned cost model trains on.
+// one LZSS chunk or one Deflate stream; every codec but Deflate has a
+// warp-level decoder (brle_warp.cuh, rlev1.cuh, rlev2.cuh, lzss.cuh), and a
+// Deflate stream is decoded by the whole block (inflate_block.cuh), so a
+// single kernel can run them all.  Tasks come from a global atomic counter
+// over an order array (dynamic: with tasks sorted longest-first this is LPT
+// list scheduling) or from the static mapping task i -> warp i mod W.
+// In a dynamic launch every warp takes its own tasks, until one takes a
+// Deflate task or sees one ahead (31 samples of the part of the queue that the
+// blocks will take next): then the block's warps finish what they have and the
+// Deflate stream is decoded.  While Deflate tasks lie ahead the block takes one
+// task at a time, so that no block collects several of the largest tasks and
+// runs them one after another; a task that is no Deflate task after all lets
+// all warps go on.
+// A Deflate stream on one warp (one lane decoding) set the makespan: 256 MiB
+// in 1024 items, the largest stream 1.7 MB, longest first: 16.1 -> 1.9 ms; with
+// four warps a block and stream 3.0 ms (the largest stream alone takes 2.9).
+// Per-task %globaltimer start/end stamps (optional) are the measurements the
+// learned cost model trains on.
 #include "brle_warp.cuh"
-#include "inflate.cuh"
+#include "inflate_block.cuh"
 #include "lzss.cuh"
 #include "rlev1.cuh"
 #include "rlev2.cuh"
@@ -19,24 +30,31 @@
 namespace gd {
 namespace batch {
 
-constexpr int WPB = 4;  // warps per block
-// Deflate workspace of a batch warp: a 4 KiB output window (nearer copies
-// from shared memory, farther ones from the output), a 1 KiB input ring, an
-// 8-bit distance table and batches of 512 literals / 64 commands (the
-// standalone kernels use up to 32 KiB, 8 KiB, 10 bits, 2048 / 256); the
-// largest codec workspace sets every warp's, so it is kept small.
-using BatchInflSmem = infl::WarpSmemT<4096, 1, 1024, 8, 512, 64>;
-
 __host__ __device__ constexpr uint32_t warp_smem_bytes(uint32_t max_lane) {
     // union of the per-codec warp workspaces
-    uint32_t a = (uint32_t)sizeof(BatchInflSmem);
     uint32_t b = lzss::WARP_SMEM;
     uint32_t c = (uint32_t)sizeof(SegTable) + ((max_lane + 15u) & ~15u) + 160u + (uint32_t)sizeof(rlev2::WarpRuns);
     uint32_t d = brlew::WARP_SMEM;
-    uint32_t m = a > b ? a : b;
-    m = m > c ? m : c;
+    uint32_t m = b > c ? b : c;
     m = m > d ? m : d;
     return (m + 15u) & ~15u;
+}
+
+// A block's warps, and its workspace for a Deflate stream.  Eight warps decode
+// a stream in 0.65 of four warps' time; four are for lane streams so long that
+// eight workspaces leave room for less than two blocks on an SM.
+struct Wide {
+    static constexpr uint32_t WPB = 8, BPS = 2;
+    using Infl = inflb::Smem<8, 32768, 2048, 16224>;
+};
+struct Narrow {
+    static constexpr uint32_t WPB = 4, BPS = 4;
+    using Infl = inflb::Smem<4, 16384, 2048, 8032>;
+};
+template <class C>
+constexpr uint32_t block_smem_bytes(uint32_t max_lane) {
+    const uint32_t w = C::WPB * warp_smem_bytes(max_lane), i = (uint32_t)sizeof(typename C::Infl);
+    return w > i ? w : i;
 }
 
 __device__ __forceinline__ uint64_t globaltimer() {
@@ -116,53 +134,150 @@ __device__ uint32_t run_task(const gd_task& t, uint32_t max_lane, uint8_t* ws) {
         case GD_CODEC_LZSS:
             if (t.dst_len != t.chunk_size || (reinterpret_cast<uintptr_t>(t.dst) & 3u)) return ST_INVALID;
             return lzss::chunk_warp(t.src, t.src_len, t.col_len, t.col_map, t.chunk_size, t.dst, ws);
-        case GD_CODEC_DEFLATE: {
-            if (t.src_len > 0xffffffffull || t.dst_len > 0xffffffffull) return ST_INVALID;
-            uint32_t fin = 0;
-            const uint32_t e = infl::stream_warp<4096, 1024, 8, 512, 64>(t.src, (uint32_t)t.src_len, t.dst,
-                                                                     (uint32_t)t.dst_len, (int)t.param,
-                                                                     *reinterpret_cast<BatchInflSmem*>(ws), &fin);
-            return (e == ST_OK && fin != (uint32_t)t.dst_len) ? (uint32_t)ST_CORRUPT : e;
-        }
         default:
             return ST_UNSUPPORTED;
     }
 }
 
-__global__ void __launch_bounds__(WPB * 32) batch_kernel(const gd_task* __restrict__ tasks, uint32_t n,
-                                                        const uint32_t* __restrict__ order, uint32_t* counter,
-                                                        int dynamic, uint32_t max_lane, uint32_t ws_bytes,
-                                                        uint32_t* __restrict__ status,
-                                                        uint64_t* __restrict__ timing) {
+// A Deflate task, by the whole block.
+template <class C>
+__device__ uint32_t deflate_task(const gd_task& t, uint8_t* smem) {
+    if (t.src_len > 0xffffffffull || t.dst_len > 0xffffffffull) return ST_INVALID;
+    uint32_t fin = 0;
+    const uint32_t e = inflb::stream_block(t.src, (uint32_t)t.src_len, t.dst, (uint32_t)t.dst_len, (int)t.param,
+                                           *reinterpret_cast<typename C::Infl*>(smem), &fin);
+    return (e == ST_OK && fin != (uint32_t)t.dst_len) ? (uint32_t)ST_CORRUPT : e;
+}
+
+template <class C>
+__global__ void __launch_bounds__(C::WPB * 32, C::BPS) batch_kernel(const gd_task* __restrict__ tasks, uint32_t n,
+                                                           const uint32_t* __restrict__ order, uint32_t* counter,
+                                                           int dynamic, uint32_t max_lane, uint32_t ws_bytes,
+                                                           uint32_t* __restrict__ status,
+                                                           uint64_t* __restrict__ timing) {
+    constexpr uint32_t WPB = C::WPB;
     extern __shared__ __align__(16) uint8_t smem[];
+    __shared__ uint32_t s_list[WPB], s_nd;  // Deflate tasks taken
+    __shared__ uint32_t s_stop, s_soon, s_end;
+    constexpr uint32_t NONE = 0xffffffffu;
     const uint32_t lane = lane_id(), wid = threadIdx.x >> 5;
-    uint8_t* ws = smem + wid * ws_bytes;
-    const uint32_t gw = blockIdx.x * WPB + wid, W = gridDim.x * WPB;
-    for (uint32_t k = 0;; ++k) {
-        uint32_t i;
-        if (dynamic) {
-            uint32_t v = 0;
-            if (lane == 0) v = atomicAdd(counter, 1u);
-            i = __shfl_sync(GD_FULL_MASK, v, 0);
-        } else {
-            i = gw + k * W;
+    auto done = [&](uint32_t ti, uint32_t e, uint64_t t0) {
+        put_status(status, ti, e);
+        if (timing) {
+            timing[2ull * ti] = t0;
+            timing[2ull * ti + 1] = globaltimer();
         }
-        if (i >= n) break;
-        const uint32_t ti = order ? order[i] : i;
-        if (ti >= n) break;  // a malformed order array ends this worker
-        const uint64_t t0 = globaltimer();
-        const gd_task t = tasks[ti];
-        const uint32_t e = run_task(t, max_lane, ws);
-        __syncwarp();
-        const uint64_t t1 = globaltimer();
-        if (lane == 0) {
-            put_status(status, ti, e);
-            if (timing) {
-                timing[2ull * ti] = t0;
-                timing[2ull * ti + 1] = t1;
+    };
+    // task of queue place j; NONE past the end, or for a malformed order array
+    auto look = [&](uint32_t j, bool& defl) -> uint32_t {
+        uint32_t ti = NONE;
+        if (j < n) ti = order ? order[j] : j;
+        if (ti >= n) ti = NONE;
+        defl = ti != NONE && tasks[ti].codec == GD_CODEC_DEFLATE;
+        return ti;
+    };
+    // the next task of the queue, for the calling warp; soon: a Deflate task
+    // lies in the part of the queue that the blocks will take next
+    auto pop = [&](bool& defl, bool& soon) -> uint32_t {
+        uint32_t i = 0;
+        if (lane == 0) i = atomicAdd(counter, 1u);
+        i = __shfl_sync(GD_FULL_MASK, i, 0);
+        bool d;
+        const uint32_t ti = __shfl_sync(GD_FULL_MASK, look(i + lane * (gridDim.x * WPB / 16u), d), 0);
+        const uint32_t m = __ballot_sync(GD_FULL_MASK, d);
+        defl = m & 1u;
+        soon = (m >> 1) != 0;
+        return ti;
+    };
+    if (threadIdx.x == 0) s_soon = 1;
+    for (uint32_t k = 0;; ++k) {
+        uint32_t first = NONE;  // warp 0: a task in hand
+        if (wid == 0) {
+            uint32_t nd = 0, end = !dynamic && (blockIdx.x + k * gridDim.x) * WPB >= n;
+            if (dynamic && s_soon) {
+                bool defl, soon;
+                first = pop(defl, soon);
+                __syncwarp();
+                end = first == NONE;
+                nd = defl;
+                if (lane == 0) {
+                    s_list[0] = first;
+                    s_soon = soon;
+                }
+            }
+            if (lane == 0) {
+                s_nd = nd;
+                s_end = end;
+                s_stop = 0;
             }
         }
+        __syncthreads();
+        if (!s_end && !s_nd) {
+            for (;;) {
+                bool defl = false, soon = false;
+                uint32_t ti = first;
+                first = NONE;
+                if (!dynamic) {
+                    ti = look((blockIdx.x + k * gridDim.x) * WPB + wid, defl);
+                } else if (ti == NONE) {
+                    if (*(volatile uint32_t*)&s_stop) break;
+                    ti = pop(defl, soon);
+                    if (ti == NONE && lane == 0) s_end = 1;
+                    if (soon && lane == 0) s_soon = 1;
+                }
+                if (ti != NONE && !defl) {
+                    const uint64_t t0 = globaltimer();
+                    const gd_task t = tasks[ti];
+                    const uint32_t e = run_task(t, max_lane, smem + wid * ws_bytes);
+                    __syncwarp();
+                    if (lane == 0) done(ti, e, t0);
+                } else if (ti != NONE && lane == 0) {
+                    s_list[atomicAdd(&s_nd, 1u)] = ti;
+                }
+                if (!dynamic || ti == NONE || defl || soon) {
+                    if (lane == 0) *(volatile uint32_t*)&s_stop = 1;
+                    break;
+                }
+            }
+        }
+        __syncthreads();
+        const uint32_t nd = s_nd, end = s_end;
+        for (uint32_t w = 0; w < nd; ++w) {
+            const uint32_t ti = s_list[w];
+            const uint64_t t0 = globaltimer();
+            const gd_task t = tasks[ti];
+            const uint32_t e = deflate_task<C>(t, smem);
+            if (threadIdx.x == 0) done(ti, e, t0);
+        }
+        if (end) break;
+        __syncthreads();  // the shared words are set for the next turn
     }
+}
+
+using Kernel = void (*)(const gd_task*, uint32_t, const uint32_t*, uint32_t*, int, uint32_t, uint32_t, uint32_t*,
+                        uint64_t*);
+struct Launch {
+    Kernel kern;
+    uint32_t grid, threads, smem, ws;
+};
+
+// The kernel and its launch shape.
+constexpr uint32_t MAX_SMEM = 220 * 1024;  // a block's workspace, at most
+template <class C>
+Launch shape_of(uint32_t max_lane, uint32_t blocks_per_sm) {
+    Launch l{batch_kernel<C>, 0, C::WPB * 32, block_smem_bytes<C>(max_lane), warp_smem_bytes(max_lane)};
+    cudaFuncSetAttribute(l.kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)l.smem);
+    int dev = 0, sms = 148, occ = 1;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, l.kern, (int)l.threads, l.smem);
+    if (occ < 1) occ = 1;
+    l.grid = (uint32_t)sms * (blocks_per_sm && blocks_per_sm < (uint32_t)occ ? blocks_per_sm : (uint32_t)occ);
+    return l;
+}
+inline Launch shape(uint32_t max_lane, uint32_t blocks_per_sm) {
+    return block_smem_bytes<Wide>(max_lane) <= 110 * 1024 ? shape_of<Wide>(max_lane, blocks_per_sm)
+                                                          : shape_of<Narrow>(max_lane, blocks_per_sm);
 }
 
 }  // namespace batch
@@ -175,34 +290,19 @@ extern "C" gd_status_t gd_batch_decode(const gd_task* d_tasks, uint32_t n_tasks,
     using namespace gd::batch;
     if (n_tasks == 0) return GD_OK;
     if (!d_tasks || (dynamic && !d_counter)) return GD_ERR_INVALID_ARG;
-    const uint32_t ws = warp_smem_bytes(max_lane_bytes);
-    const uint32_t smem = WPB * ws;
-    if (smem > 220 * 1024) return GD_ERR_UNSUPPORTED;
+    const Launch l = shape(max_lane_bytes, blocks_per_sm);
+    if (l.smem > MAX_SMEM) return GD_ERR_UNSUPPORTED;
     cudaStream_t s = (cudaStream_t)stream;
-    cudaFuncSetAttribute(batch_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-    int dev = 0, sms = 148, occ = 1;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, batch_kernel, WPB * 32, smem);
-    if (occ < 1) occ = 1;
-    const uint32_t bps = blocks_per_sm ? (blocks_per_sm < (uint32_t)occ ? blocks_per_sm : (uint32_t)occ) : (uint32_t)occ;
     if (dynamic && cudaMemsetAsync(d_counter, 0, sizeof(uint32_t), s) != cudaSuccess) return GD_ERR_CUDA;
-    batch_kernel<<<bps * (uint32_t)sms, WPB * 32, smem, s>>>(d_tasks, n_tasks, d_order, d_counter, dynamic,
-                                                            max_lane_bytes, ws, d_status, d_timing);
+    l.kern<<<l.grid, l.threads, l.smem, s>>>(d_tasks, n_tasks, d_order, d_counter, dynamic, max_lane_bytes, l.ws,
+                                             d_status, d_timing);
     return cudaGetLastError() == cudaSuccess ? GD_OK : GD_ERR_CUDA;
 }
 
 extern "C" uint32_t gd_batch_warps(uint32_t max_lane_bytes, uint32_t blocks_per_sm) {
     using namespace gd::batch;
-    const uint32_t smem = WPB * warp_smem_bytes(max_lane_bytes);
-    cudaFuncSetAttribute(batch_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-    int dev = 0, sms = 148, occ = 1;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, batch_kernel, WPB * 32, smem);
-    if (occ < 1) occ = 1;
-    const uint32_t bps = blocks_per_sm ? (blocks_per_sm < (uint32_t)occ ? blocks_per_sm : (uint32_t)occ) : (uint32_t)occ;
-    return bps * (uint32_t)sms * WPB;
+    const Launch l = shape(max_lane_bytes, blocks_per_sm);
+    return l.grid * (l.threads / 32u);
 }
 
 // ---------------------------------------------------------------------------
@@ -330,37 +430,22 @@ extern "C" gd_status_t gd_batch_decode_lpt_noalloc(const gd_task* d_tasks, uint3
     if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return GD_ERR_CUDA;
     static std::mutex mu;
     static uint32_t* scratch_of[64] = {};
-    static int sms_of[64] = {};
     uint32_t* scratch;
-    int sms;
     {
         std::lock_guard<std::mutex> g(mu);
         if (!scratch_of[dev]) {
             void* p = nullptr;
             if (cudaGetSymbolAddress(&p, g_noalloc_scratch) != cudaSuccess || !p) return GD_ERR_CUDA;
-            int m = 0;
-            if (cudaDeviceGetAttribute(&m, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || m <= 0)
-                return GD_ERR_CUDA;
-            sms_of[dev] = m;
             scratch_of[dev] = static_cast<uint32_t*>(p);
         }
         scratch = scratch_of[dev];
-        sms = sms_of[dev];
     }
-    const uint32_t ws = warp_smem_bytes(max_lane_bytes);
-    const uint32_t smem = WPB * ws;
-    if (smem > 220 * 1024) return GD_ERR_UNSUPPORTED;
+    const Launch l = shape(max_lane_bytes, blocks_per_sm);
+    if (l.smem > MAX_SMEM) return GD_ERR_UNSUPPORTED;
     cudaStream_t s = (cudaStream_t)stream;
-    if (cudaFuncSetAttribute(batch_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess)
-        return GD_ERR_CUDA;
-    int occ = 1;
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, batch_kernel, WPB * 32, smem);
-    if (occ < 1) occ = 1;
-    const uint32_t bps = blocks_per_sm ? (blocks_per_sm < (uint32_t)occ ? blocks_per_sm : (uint32_t)occ) : (uint32_t)occ;
     lpt_sort_kernel<<<1, SORT_NT, 0, s>>>(d_cost, n_tasks, scratch);
     if (cudaGetLastError() != cudaSuccess) return GD_ERR_CUDA;
-    batch_kernel<<<bps * (uint32_t)sms, WPB * 32, smem, s>>>(d_tasks, n_tasks, scratch,
-                                                            scratch + NOALLOC_MAX_TASKS + NBUCKET, 1,
-                                                            max_lane_bytes, ws, d_status, nullptr);
+    l.kern<<<l.grid, l.threads, l.smem, s>>>(d_tasks, n_tasks, scratch, scratch + NOALLOC_MAX_TASKS + NBUCKET, 1,
+                                             max_lane_bytes, l.ws, d_status, nullptr);
     return cudaGetLastError() == cudaSuccess ? GD_OK : GD_ERR_CUDA;
 }

@@ -52,7 +52,7 @@ template <class Chunks, uint32_t WIN, int NP, uint32_t RB = IRING, uint32_t DB =
 __global__ void __launch_bounds__(NP * 64) inflate_pair_kernel(Chunks ch, uint32_t n_chunks, int zlib_hdr,
                                                               const uint32_t* __restrict__ order,
                                                               uint32_t spin_limit, uint32_t writer_stop) {
-    using SmemT = WarpSmemT<WIN, 2, RB, DB, NL, NC>;
+    using SmemT = WarpSmemT<WIN, RB, DB, NL, NC>;
     extern __shared__ __align__(16) uint8_t smem_raw[];
     const uint32_t wid = threadIdx.x >> 5, pair = wid >> 1;
     const uint32_t slot = blockIdx.x * NP + pair;
@@ -81,7 +81,7 @@ __global__ void __launch_bounds__(NP * 64) inflate_pair_kernel(Chunks ch, uint32
         return;
     }
     uint32_t fin = 0;
-    err = stream_warp_impl<WIN, 2, RB, DB, NL, NC>(src, (uint32_t)clen64, dst, (uint32_t)olen64, zlib_hdr, S, &fin,
+    err = stream_warp_impl<WIN, RB, DB, NL, NC>(src, (uint32_t)clen64, dst, (uint32_t)olen64, zlib_hdr, S, &fin,
                                                    spin_limit);
     if (err == ST_OK && Chunks::exact && fin != (uint32_t)olen64) err = ST_CORRUPT;
     if (lane_id() == 0) ch.put(chunk, err, err == ST_OK ? fin : 0);
@@ -127,7 +127,7 @@ template <class Chunks, uint32_t WIN, int NP, uint32_t RB = gd::infl::IRING, uin
           uint32_t NL = gd::infl::NLIT, uint32_t NC = gd::infl::NCMD>
 gd_status_t launch_pair(const Chunks& ch, uint32_t n, int zlib_hdr, const uint32_t* order, cudaStream_t s) {
     using namespace gd::infl;
-    const uint32_t smem = NP * (uint32_t)sizeof(WarpSmemT<WIN, 2, RB, DB, NL, NC>);
+    const uint32_t smem = NP * (uint32_t)sizeof(WarpSmemT<WIN, RB, DB, NL, NC>);
     auto kern = inflate_pair_kernel<Chunks, WIN, NP, RB, DB, NL, NC>;
     static bool attr_set = false;  // benign race: the attribute call is idempotent
     if (!attr_set) {

@@ -1,25 +1,24 @@
-// inflate.cuh -- warp-level Deflate / zlib / gzip inflate for sm_100a
-// (shared by the plain kernels in inflate.cu and the batched decoder).
+// inflate.cuh -- Deflate / zlib / gzip inflate by a warp pair (sm_100a), the
+// kernel that GD_TUNE_INFLATE_VARIANT 6 and 12 choose; a block per stream
+// (inflate_block.cuh) is the default and 4 to 9 times faster.
 //
 // Replaces the reference's deflate::inflate / inflate_shared
 // (include/zlib/zlib.h:832-962): there one lane per chunk decodes codes
 // bit-serially from global-memory trees (zlib.h:233-266) and a writer warp
 // copies back-references; stored blocks are dropped (zlib.h:532-543).
 //
-// Here one warp owns a chunk and alternates two phases:
-//   decode  -- lane 0 reads the bit stream from a shared-memory input ring and
+// Here a decoder and a writer warp own a chunk:
+//   decoder -- lane 0 reads the bit stream from a shared-memory input ring and
 //              decodes symbols with 10-bit lookup tables (longer codes fall
 //              back to a canonical count/symbol walk), appending commands
 //              (literal runs, (length, distance) copies, stored blocks) to a
-//              shared command buffer;
-//   execute -- all 32 lanes write the commands to the output: literal runs
-//              and stored data as coalesced byte stores, copies in 32-byte
-//              waves (distance >= 32: each wave reads bytes written by earlier
-//              waves; distance < 32: the period-`distance` pattern is read
-//              from before the copy).  The warp also refills the input ring.
-//              With a window (WIN > 0) the last 32 KiB of output are kept in
-//              shared memory and copies read only there.
-// Dynamic tables are rebuilt per block; table fills are spread over the warp.
+//              shared command buffer; the warp refills the ring and builds
+//              the tables;
+//   writer  -- all 32 lanes write a batch of commands to the output while the
+//              next is decoded: literal runs and stored data as coalesced byte
+//              stores, copies in 128- or 32-byte waves (distance >= that),
+//              nearer ones as the period-`distance` pattern.
+// The last WIN bytes of output are kept in shared memory for the copies.
 // Every read is bounded by the chunk's compressed size and every write by its
 // output size; malformed input yields GD_ERR_CORRUPT / GD_ERR_OVERRUN.
 #pragma once
@@ -70,135 +69,26 @@ struct BatchT {
 };
 using Batch = BatchT<NLIT, NCMD>;
 
-// Per-stream shared state.  WIN > 0: the last WIN output bytes are kept in a
+// Per-stream shared state.  The last WIN output bytes are kept in a
 // shared-memory window (a power of two; with 32768, the Deflate window, no
-// back-reference reads global memory, with less only the farther ones do);
-// WIN = 0: copies read the output already written to global memory (a
-// smaller footprint, for kernels that run other decoders beside this one).  NB = 1: one warp decodes and
-// executes; NB = 2: a decoder warp fills batch k+1 while a writer warp
-// executes batch k.
+// back-reference reads global memory, with less only the farther ones do).
+// The decoder warp fills batch k+1 while the writer warp executes batch k.
 // RB: input ring bytes; DB: distance lookup bits; NL / NC: literal bytes and
 // commands per batch (smaller values for kernels that run many warps).
-template <uint32_t WIN, int NB = 1, uint32_t RB = IRING, uint32_t DB = LBITS, uint32_t NL = NLIT, uint32_t NC = NCMD>
+template <uint32_t WIN, uint32_t RB = IRING, uint32_t DB = LBITS, uint32_t NL = NLIT, uint32_t NC = NCMD>
 struct alignas(16) WarpSmemT {
-    uint8_t win[WIN ? WIN : 16];
+    uint8_t win[WIN];
     uint8_t ring[RB];
     HuffT<LBITS> lit;
     HuffT<DB> dist;
     uint8_t lens[320];
     uint8_t cl_tmp[320];   // code lengths while a dynamic header is read
     uint16_t offs[16];     // canonical code offsets (build_huff)
-    BatchT<NL, NC> bt[NB];
+    BatchT<NL, NC> bt[2];
     // decoder state shared between lane 0 and the warp
     uint32_t status, done;
     uint32_t produced, consumed;  // pair hand-off counters
 };
-using WarpSmem = WarpSmemT<0, 1>;
-
-// Windowless form: copies read the output already written (global memory).
-// Up to 4 consecutive commands whose sources all lie before the first of
-// them -- literal runs, and copies of at most 128 bytes whose distance
-// exceeds their offset into the group plus their length -- are executed
-// together: every lane issues all of its loads (4 bytes per command) before
-// any store, so the group pays one memory latency instead of one per
-// command.  Other commands run one at a time.
-template <class BatchType>
-static __device__ __forceinline__ void execute_batch_out(const BatchType& B, uint32_t pos,
-                                                         const uint8_t* __restrict__ src,
-                                                         uint8_t* __restrict__ dst) {
-    const uint32_t lane = lane_id();
-    const uint32_t nc = B.n_cmd;
-    uint32_t c = 0;
-    while (c < nc) {
-        uint32_t tg[4], ag[4], ng[4];
-#pragma unroll
-        for (uint32_t i = 0; i < 4; ++i) {
-            const bool ok = c + i < nc;
-            tg[i] = ok ? B.cmd_t[c + i] : (uint32_t)C_STORED;
-            ag[i] = ok ? B.cmd_a[c + i] : 0u;
-            ng[i] = ok ? B.cmd_b[c + i] : 0u;
-        }
-        uint32_t g = 0, off = 0;
-#pragma unroll
-        for (uint32_t i = 0; i < 4; ++i) {
-            const bool fits = ng[i] <= 128u && (tg[i] == C_LIT || (tg[i] == C_COPY && ag[i] >= off + ng[i]));
-            if (g == i && fits) {
-                g = i + 1;
-                off += ng[i];
-            }
-        }
-        if (g >= 2) {
-            uint8_t v[4][4];
-            uint32_t o = 0;
-#pragma unroll
-            for (uint32_t i = 0; i < 4; ++i) {
-#pragma unroll
-                for (uint32_t w = 0; w < 4; ++w) {
-                    const uint32_t k = lane + 32u * w;
-                    v[i][w] = 0;
-                    if (i < g && k < ng[i])
-                        v[i][w] = tg[i] == C_LIT ? B.lits[ag[i] + k] : dst[pos + o - ag[i] + k];
-                }
-                o += i < g ? ng[i] : 0u;
-            }
-            o = 0;
-#pragma unroll
-            for (uint32_t i = 0; i < 4; ++i) {
-#pragma unroll
-                for (uint32_t w = 0; w < 4; ++w) {
-                    const uint32_t k = lane + 32u * w;
-                    if (i < g && k < ng[i]) dst[pos + o + k] = v[i][w];
-                }
-                o += i < g ? ng[i] : 0u;
-            }
-            pos += o;
-            c += g;
-            __syncwarp();
-            continue;
-        }
-        const uint32_t t = tg[0], a = ag[0], n = ng[0];
-        uint8_t* d = dst + pos;
-        if (t == C_LIT) {
-            for (uint32_t k = lane; k < n; k += 32) d[k] = B.lits[a + k];
-        } else if (t == C_STORED) {
-            const uint8_t* s = src + a;
-            for (uint32_t k = lane; k < n; k += 32) d[k] = s[k];
-        } else {
-            const uint8_t* s = d - a;
-            if (a >= 128) {  // 128-byte waves: one latency per 128 bytes
-                for (uint32_t k0 = 0; k0 < n; k0 += 128) {
-                    uint8_t v[4];
-#pragma unroll
-                    for (uint32_t w = 0; w < 4; ++w) {
-                        const uint32_t k = k0 + lane + 32u * w;
-                        v[w] = k < n ? s[k] : (uint8_t)0;
-                    }
-                    __syncwarp();
-#pragma unroll
-                    for (uint32_t w = 0; w < 4; ++w) {
-                        const uint32_t k = k0 + lane + 32u * w;
-                        if (k < n) d[k] = v[w];
-                    }
-                    __syncwarp();
-                }
-            } else if (a >= 32) {
-                for (uint32_t k0 = 0; k0 < n; k0 += 32) {
-                    const uint32_t k = k0 + lane;
-                    uint8_t v = 0;
-                    if (k < n) v = s[k];
-                    __syncwarp();
-                    if (k < n) d[k] = v;
-                    __syncwarp();
-                }
-            } else {
-                for (uint32_t k = lane; k < n; k += 32) d[k] = s[k % a];
-            }
-        }
-        pos += n;
-        ++c;
-        __syncwarp();
-    }
-}
 
 // Write batch B (output starting at pos) with the calling warp.
 template <uint32_t WIN, class BatchType>
@@ -206,10 +96,6 @@ static __device__ __forceinline__ void execute_batch(const BatchType& B, uint32_
                                                      const uint8_t* __restrict__ src, uint8_t* __restrict__ dst) {
     const uint32_t lane = lane_id();
     const uint32_t nc = B.n_cmd;
-    if constexpr (WIN == 0) {
-        execute_batch_out(B, pos, src, dst);
-        return;
-    }
     // the next command's fields are loaded before the current one is written
     uint32_t tn = nc ? B.cmd_t[0] : 0u, an = nc ? B.cmd_a[0] : 0u, nn = nc ? B.cmd_b[0] : 0u;
     for (uint32_t c = 0; c < nc; ++c) {
@@ -220,7 +106,7 @@ static __device__ __forceinline__ void execute_batch(const BatchType& B, uint32_
             nn = B.cmd_b[c + 1];
         }
         uint8_t* d = dst + pos;
-        if constexpr (WIN != 0) {
+        {
             // every output byte also goes to the window; copies read it there
             constexpr uint32_t M = WIN - 1;
             if (t == C_LIT) {
@@ -448,19 +334,18 @@ static __device__ bool build_huff(HuffT<BITS>* h, const uint8_t* lens, uint32_t 
 // olen bytes; hdr: 0 raw deflate, 1 zlib, 2 gzip; S: this warp's shared
 // state.  Returns a gd status (same on every lane); *written = bytes output.
 // stream_warp_impl is inlined into the caller, so the compiler sees that S is
-// shared memory and uses shared-memory loads and stores throughout;
-// stream_warp is the out-of-line form for kernels that run several decoders.
-// NB = 2 (decoder of a pair): instead of executing a batch, hand it to the
-// writer warp (see stream_pair_writer); S.produced / S.consumed must be 0.
-template <uint32_t WIN, int NB = 1, uint32_t RB = IRING, uint32_t DB = LBITS, uint32_t NL = NLIT, uint32_t NC = NCMD>
+// shared memory and uses shared-memory loads and stores throughout.
+// Batches are handed to the writer warp (see stream_pair_writer); S.produced
+// and S.consumed must be 0.
+template <uint32_t WIN, uint32_t RB = IRING, uint32_t DB = LBITS, uint32_t NL = NLIT, uint32_t NC = NCMD>
 static __device__ __forceinline__ uint32_t stream_warp_impl(const uint8_t* __restrict__ src, uint32_t clen,
                                                             uint8_t* __restrict__ dst, uint32_t olen, int zlib_hdr,
-                                                            WarpSmemT<WIN, NB, RB, DB, NL, NC>& S, uint32_t* written,
+                                                            WarpSmemT<WIN, RB, DB, NL, NC>& S, uint32_t* written,
                                                             uint32_t spin_limit = PAIR_SPIN_LIMIT) {
     static_assert(RB >= 1024 && (RB & (RB - 1)) == 0, "input ring: a power of two >= 1 KiB");
     // a window below the Deflate window's 32 KiB serves the nearer copies;
     // the executor reads farther ones from the output
-    static_assert(WIN == 0 || (WIN >= 2048 && (WIN & (WIN - 1)) == 0), "window: 0 or a power of two >= 2 KiB");
+    static_assert(WIN >= 2048 && (WIN & (WIN - 1)) == 0, "window: a power of two >= 2 KiB");
     const uint32_t lane = lane_id();
     uint32_t err = ST_OK;
     // input ring: compressed byte i (chunk-relative) at ring[(i + sh) % RB];
@@ -625,13 +510,11 @@ static __device__ __forceinline__ uint32_t stream_warp_impl(const uint8_t* __res
     // main loop ------------------------------------------------------------
     uint32_t kb = 0;  // batches handed off (pairs: the buffer is bt[kb & 1])
     while (err == ST_OK) {
-        auto& BT = S.bt[NB == 2 ? (kb & 1u) : 0u];
+        auto& BT = S.bt[kb & 1u];
         // pairs: the buffer's previous batch (kb - 2) must have been executed
-        if constexpr (NB == 2) {
-            if (kb >= 2 && !pair_wait(&S.consumed, kb - 1, spin_limit)) {
-                err = ST_TIMEOUT;
-                break;
-            }
+        if (kb >= 2 && !pair_wait(&S.consumed, kb - 1, spin_limit)) {
+            err = ST_TIMEOUT;
+            break;
         }
         // ---- refill input for the decoder (warp) ----
         uint32_t inpos_b = __shfl_sync(GD_FULL_MASK, inpos, 0);
@@ -975,18 +858,14 @@ static __device__ __forceinline__ uint32_t stream_warp_impl(const uint8_t* __res
             for (int o = 16; o; o >>= 1) tot += __shfl_xor_sync(GD_FULL_MASK, tot, o);
             pos -= tot;
         }
-        if constexpr (NB == 2) {
-            if (lane == 0) {
-                BT.pos0 = pos;
-                BT.last = 0;
-            }
-            pair_post(&S.produced, kb + 1);
-            ++kb;
-        } else {
-            execute_batch<WIN>(BT, pos, S.win, src, dst);
+        if (lane == 0) {
+            BT.pos0 = pos;
+            BT.last = 0;
         }
+        pair_post(&S.produced, kb + 1);
+        ++kb;
     }
-    if constexpr (NB == 2) {  // the final (empty) hand-off
+    {  // the final (empty) hand-off
         if (err != ST_TIMEOUT && kb >= 2 && !pair_wait(&S.consumed, kb - 1, spin_limit)) err = ST_TIMEOUT;
         auto& BT = S.bt[kb & 1u];
         if (lane == 0) {
@@ -1000,21 +879,14 @@ static __device__ __forceinline__ uint32_t stream_warp_impl(const uint8_t* __res
     return __shfl_sync(GD_FULL_MASK, err, 0);
 }
 
-template <uint32_t WIN, uint32_t RB = IRING, uint32_t DB = LBITS, uint32_t NL = NLIT, uint32_t NC = NCMD>
-static __device__ __noinline__ uint32_t stream_warp(const uint8_t* __restrict__ src, uint32_t clen,
-                                                    uint8_t* __restrict__ dst, uint32_t olen, int zlib_hdr,
-                                                    WarpSmemT<WIN, 1, RB, DB, NL, NC>& S, uint32_t* written) {
-    return stream_warp_impl<WIN, 1, RB, DB, NL, NC>(src, clen, dst, olen, zlib_hdr, S, written);
-}
-
 // Writer warp of a pair: executes batch k while the decoder warp (running
-// stream_warp_impl<WIN, 2> on the same S) decodes batch k+1.  The decoder's
+// stream_warp_impl on the same S) decodes batch k+1.  The decoder's
 // last hand-off is an empty batch marked last (also after an error).
 // Returns GD_ERR_TIMEOUT if a wait expired, else OK.  stop_after > 0 (a test
 // setting) makes the writer leave after that many batches without posting
 // more, so that the decoder's bounded wait is exercised.
 template <uint32_t WIN, uint32_t RB = IRING, uint32_t DB = LBITS, uint32_t NL = NLIT, uint32_t NC = NCMD>
-static __device__ __forceinline__ uint32_t stream_pair_writer(WarpSmemT<WIN, 2, RB, DB, NL, NC>& S,
+static __device__ __forceinline__ uint32_t stream_pair_writer(WarpSmemT<WIN, RB, DB, NL, NC>& S,
                                                               const uint8_t* __restrict__ src,
                                                               uint8_t* __restrict__ dst, uint32_t spin_limit,
                                                               uint32_t stop_after) {
