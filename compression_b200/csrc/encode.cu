@@ -3,17 +3,11 @@
 // The writer side of the two interleaved integer containers
 // (rle_v1::compress_gpu, include/rle_v1/rlev1.h:25-97;
 // rlev2::compress_gpu_transpose, include/rlev2/encoder_trans.h:428-537),
-// producing the same bytes as the host encoders (both run the lane encoders
-// of lane_enc.h).  Three launches on one stream:
-//   1. the lane streams: RLE v1, lane_encode_kernel: a warp per chunk, a
-//      thread per lane stream.  Each thread gathers its lane's values straight
-//      from the column (COMP_COL_LEN-byte slices at a 32-slice stride) and runs
-//      the lane encoder into its own scratch slot, buffering 4 bytes in a
-//      register so the scratch is written in whole words (the literal-count
-//      byte written back later is a byte store or a register edit).  RLE v2: a
-//      warp per lane stream (rlev2_enc.cuh), then a warp per chunk sums the
-//      padded word counts into the block size (lane_encode_kernel does that
-//      itself);
+// producing the same bytes as the host encoders (gd_encode.cpp, lane_enc.h).
+// Launches on one stream:
+//   1. the lane streams, a warp each (rlev1_enc.cuh, rlev2_enc.cuh), into
+//      scratch slots; then a warp per chunk sums the padded word counts into
+//      the chunk's block size;
 //   2. offsets_kernel: one block turns the block sizes into blk_off;
 //   3. interleave_kernel: row k = one word of every lane longer than 4k bytes,
 //      in lane order, through the same segment table the decoders read with
@@ -22,12 +16,13 @@
 #include "gd_common.cuh"
 #include "interleave.cuh"
 #include "lane_enc.h"
+#include "rlev1_enc.cuh"
 #include "rlev2_enc.cuh"
 
 namespace gd {
 namespace encd {
 
-constexpr int NT = 128;  // threads per block (4 chunks per block in launch 1)
+constexpr int NT = 128;  // threads per block
 
 // Byte sink over one lane's scratch slot (cap bytes, a multiple of 4).
 struct DevSink {
@@ -55,48 +50,6 @@ struct DevSink {
         if ((n & 3u) && n < cap) w[n >> 2] = cur;
     }
 };
-
-// RLE v1 lane t: value e is element (e / wil) * 32 * wil + t * wil + e % wil
-// of the chunk (encoder.h:139-153); elements past the input are zero.
-template <typename T>
-struct V1Vals {
-    const T* base;
-    uint64_t avail;
-    uint32_t t, wil;
-    __device__ __forceinline__ T operator[](uint64_t e) const {
-        const uint32_t q = (uint32_t)e / wil, r = (uint32_t)e - q * wil;
-        const uint64_t idx = (uint64_t)q * 32u * wil + (uint64_t)t * wil + r;
-        return idx < avail ? base[idx] : (T)0;
-    }
-};
-
-// RLE v1: blk_size[c] gets chunk c's block size (the launch passes blk_off + 1).
-template <typename T>
-__global__ void __launch_bounds__(NT) lane_encode_kernel(const uint8_t* __restrict__ in, uint64_t n_bytes,
-                                                         uint32_t n_chunks, uint64_t chunk_size, uint32_t wil,
-                                                         uint8_t* __restrict__ scratch, uint32_t lane_cap,
-                                                         uint64_t* __restrict__ col_len,
-                                                         uint64_t* __restrict__ blk_size,
-                                                         uint32_t* __restrict__ status) {
-    const uint32_t c = (blockIdx.x * NT + threadIdx.x) >> 5;
-    const uint32_t t = lane_id();
-    if (c >= n_chunks) return;  // warp-uniform
-    const uint64_t cb = (uint64_t)c * chunk_size;
-    const uint64_t have = n_bytes > cb ? (n_bytes - cb < chunk_size ? n_bytes - cb : chunk_size) : 0;
-    DevSink s{reinterpret_cast<uint32_t*>(scratch + ((uint64_t)c * 32u + t) * lane_cap), 0u, lane_cap, 0u};
-    const V1Vals<T> v{reinterpret_cast<const T*>(in + cb), have / sizeof(T), t, wil};
-    enc::rlev1_encode_lane<T>(v, chunk_size / 32u / sizeof(T), s);
-    s.flush();
-    const bool over = s.n > lane_cap;
-    const uint32_t len = over ? 0u : s.n;
-    col_len[(uint64_t)c * 32u + t] = len;
-    const uint32_t words = __reduce_add_sync(GD_FULL_MASK, (len + 3u) >> 2);
-    const bool bad = __any_sync(GD_FULL_MASK, over);
-    if (t == 0) {
-        blk_size[c] = ((uint64_t)words * 4u + 127u) & ~127ull;
-        put_status(status, c, bad ? (uint32_t)ST_OVERRUN : (uint32_t)ST_OK);
-    }
-}
 
 // blk_off[1..n] hold block sizes on entry and their inclusive prefix sums on
 // exit; blk_off[0] = 0.  One block of 1024 threads, each over a contiguous
@@ -442,10 +395,10 @@ extern "C" gd_status_t gd_rlev1_encode_device(const uint8_t* d_in, uint64_t n_by
     const uint32_t wil = comp_col_len / elem_bytes;
     cudaStream_t s = (cudaStream_t)stream;
     const uint64_t nc = (n_bytes + chunk_size - 1) / chunk_size;
-    auto kern = elem_bytes == 4 ? lane_encode_kernel<uint32_t> : lane_encode_kernel<uint64_t>;
-    kern<<<(uint32_t)((nc + NT / 32 - 1) / (NT / 32)), NT, 0, s>>>(d_in, n_bytes, (uint32_t)nc, chunk_size, wil,
-                                                                   d_scratch, (uint32_t)cap, d_col_len, d_blk_off + 1,
-                                                                   d_status);
+    auto kern = elem_bytes == 4 ? rlev1_encode_kernel<uint32_t> : rlev1_encode_kernel<uint64_t>;
+    kern<<<(uint32_t)((nc * 32u + V1_WPB - 1) / V1_WPB), V1_WPB * 32, 0, s>>>(d_in, n_bytes, nc * 32u, chunk_size, wil,
+                                                                              d_scratch, (uint32_t)cap, d_col_len);
+    lane_sizes_kernel<<<(uint32_t)((nc + 3) / 4), 128, 0, s>>>((uint32_t)nc, d_col_len, d_blk_off + 1, d_status);
     return finish(nc, d_scratch, cap, d_data, d_blk_off, d_col_len, nullptr, s);
 }
 
