@@ -24,33 +24,6 @@ namespace encd {
 
 constexpr int NT = 128;  // threads per block
 
-// Byte sink over one lane's scratch slot (cap bytes, a multiple of 4).
-struct DevSink {
-    uint32_t* w;
-    uint32_t n, cap, cur;  // bytes put; capacity; bytes [n & ~3, n) not yet stored
-    __device__ __forceinline__ void put(uint8_t b) {
-        cur |= (uint32_t)b << (8u * (n & 3u));
-        ++n;
-        if ((n & 3u) == 0) {
-            if (n <= cap) w[(n >> 2) - 1] = cur;
-            cur = 0;
-        }
-    }
-    __device__ __forceinline__ uint32_t size() const { return n; }
-    __device__ __forceinline__ void set(uint64_t i, uint8_t b) {
-        if (i >= (n & ~3u)) {
-            const uint32_t sh = 8u * ((uint32_t)i & 3u);
-            cur = (cur & ~(0xffu << sh)) | ((uint32_t)b << sh);
-        } else if (i < cap) {
-            reinterpret_cast<uint8_t*>(w)[i] = b;
-        }
-    }
-    // store the last partial word (its unused bytes are zero)
-    __device__ __forceinline__ void flush() {
-        if ((n & 3u) && n < cap) w[n >> 2] = cur;
-    }
-};
-
 // blk_off[1..n] hold block sizes on entry and their inclusive prefix sums on
 // exit; blk_off[0] = 0.  One block of 1024 threads, each over a contiguous
 // range of chunks.
@@ -147,47 +120,62 @@ inline dim3 interleave_grid(uint64_t n_chunks, uint64_t lane_cap) {
 // (length - 3), offsets 1..2047 back into the column, lengths 3..34).  The
 // greedy writer takes at every position the oldest of the longest matches in
 // the 2048-byte history (find_match, lzss_gpu2.h:70-108), so a position's
-// match depends only on the position: a warp per column stages the column in
-// shared memory, indexes its 3-byte keys by hash bucket (positions ascending
-// inside a bucket), and at each token checks the bucket's candidates 32 at a
-// time, oldest first (one lane per candidate, the longest with the oldest
-// winning ties), stopping at a 34-byte match.  A per-bucket cursor drops
-// candidates older than the history as the walk advances.  Lane 0 writes the
-// tokens into the column's scratch slot.  (Finding every position's match
-// with a lane per position instead was 2.4x slower on Markov columns: their
-// candidate lists are long, and serial per lane.)
+// match depends only on the position.  A warp per column:
+//   - stages the column in shared memory and sorts its positions by a hash of
+//     their 3-byte keys, ascending inside a bucket;
+//   - marks the positions that have a match, a lane per sorted position
+//     looking back in its bucket for its key (usually the entry before);
+//   - walks the tokens: literals up to the next marked position in one step,
+//     and there the bucket's candidates 32 at a time, oldest first (one lane
+//     per candidate, compared 4 bytes at a time, the longest with the oldest
+//     winning ties), stopping at a 34-byte match;
+//   - queues tokens a lane each and writes 32 (four flag groups) together.
+// Searching at every token, literals too (64% of the benchmark's), and writing
+// each token from one lane took 88 warp instructions a token and 5.66 ms for
+// 64 MiB.  (Finding every position's match with a lane per position was 2.4x
+// slower still: the candidate lists are long, and serial per lane.)
 
 constexpr uint32_t LZ_WPB = 4;      // columns (warps) per block
 constexpr uint32_t LZ_NB = 512;     // hash buckets of 3-byte keys
-constexpr uint32_t LZ_HIST = 2048, LZ_LOOK = 512, LZ_MAXM = 34, LZ_MINM = 3;
+constexpr uint32_t LZ_HIST = 2048, LZ_MAXM = 34, LZ_MINM = 3;
+constexpr uint32_t LZ_OUT = 256;    // output bytes held back: less than 128, and the next 32 tokens
 
 __host__ __device__ constexpr uint32_t a16(uint32_t x) { return (x + 15u) & ~15u; }
-// column bytes (+64 zero pad) | positions by bucket | bucket starts | cursors
+// column bytes (+64 zero pad) | positions by bucket, also the counts before them | bucket ends | marks | output |
+// oldest candidates by bucket, where the column is longer than the history
+__host__ __device__ constexpr uint32_t lz_pos_bytes(uint32_t L) { return a16(2u * L > 4u * LZ_NB ? 2u * L : 4u * LZ_NB); }
 __host__ __device__ constexpr uint32_t lz_warp_smem(uint32_t L) {
-    return a16(L + 64u) + a16(2u * L) + a16(2u * (LZ_NB + 1u)) + a16(2u * LZ_NB);
+    return a16(L + 64u) + lz_pos_bytes(L) + a16(2u * LZ_NB) + a16(L / 8u + 8u) + LZ_OUT + (L > LZ_HIST ? a16(2u * LZ_NB) : 0u);
 }
-__device__ __forceinline__ uint32_t lz_key(const uint8_t* d, uint32_t p) {
-    return ((uint32_t)d[p] << 16) | ((uint32_t)d[p + 1] << 8) | d[p + 2];
+// the 4 bytes at p
+__device__ __forceinline__ uint32_t lz_word(const uint8_t* d, uint32_t p) {
+    const uint32_t* w = reinterpret_cast<const uint32_t*>(d) + (p >> 2);
+    return __funnelshift_r(w[0], w[1], 8u * (p & 3u));
 }
-__device__ __forceinline__ uint32_t lz_hash(uint32_t key) { return (key * 2654435761u) >> 23; }  // 9 bits
+__device__ __forceinline__ uint32_t lz_hash(uint32_t word) { return ((word & 0xffffffu) * 2654435761u) >> 23; }  // 9 bits
 
 __global__ void __launch_bounds__(LZ_WPB * 32) lzss_column_kernel(const uint8_t* __restrict__ in, uint64_t n_bytes,
                                                                   uint64_t chunk_size, uint32_t n_cols,
                                                                   uint8_t* __restrict__ scratch, uint32_t cap,
                                                                   uint32_t* __restrict__ raw_len, uint32_t wsm) {
     extern __shared__ __align__(16) uint8_t smem[];
-    const uint32_t lane = lane_id(), wid = threadIdx.x >> 5;
+    const uint32_t lane = lane_id(), wid = threadIdx.x >> 5, lt = (1u << lane) - 1u;
     const uint32_t col = blockIdx.x * LZ_WPB + wid;  // 32 * chunk + column
     if (col >= n_cols) return;                        // warp-uniform
     const uint32_t q = col & 31u;
     const uint32_t L = (uint32_t)(chunk_size / 32u);
     uint8_t* d = smem + wid * wsm;
     uint16_t* pos = reinterpret_cast<uint16_t*>(d + a16(L + 64u));
-    uint16_t* start = reinterpret_cast<uint16_t*>(reinterpret_cast<uint8_t*>(pos) + a16(2u * L));
-    uint16_t* cursor = reinterpret_cast<uint16_t*>(reinterpret_cast<uint8_t*>(start) + a16(2u * (LZ_NB + 1u)));
+    uint32_t* cnt = reinterpret_cast<uint32_t*>(pos);
+    uint16_t* end = reinterpret_cast<uint16_t*>(reinterpret_cast<uint8_t*>(pos) + lz_pos_bytes(L));
+    uint32_t* mark = reinterpret_cast<uint32_t*>(reinterpret_cast<uint8_t*>(end) + a16(2u * LZ_NB));
+    uint8_t* out = reinterpret_cast<uint8_t*>(mark) + a16(L / 8u + 8u);
+    uint16_t* oldest = reinterpret_cast<uint16_t*>(out + LZ_OUT);
+    const bool aged = L > LZ_HIST;  // candidates can leave the history
 
     // ---- the column: word k = chunk bytes [128k + 4q, +4); zero past the input ----
     const uint64_t cb = (uint64_t)(col >> 5) * chunk_size;
+#pragma unroll 4
     for (uint32_t k = lane; k < L / 4u; k += 32) {
         const uint64_t g = cb + 128ull * k + 4u * q;
         uint32_t w = 0;
@@ -199,113 +187,164 @@ __global__ void __launch_bounds__(LZ_WPB * 32) lzss_column_kernel(const uint8_t*
         }
         reinterpret_cast<uint32_t*>(d)[k] = w;
     }
-    for (uint32_t i = L + lane; i < L + 64u; i += 32) d[i] = 0;
-    for (uint32_t b = lane; b < LZ_NB; b += 32) cursor[b] = 0;
+    for (uint32_t i = L / 4u + lane; i < L / 4u + 16u; i += 32) reinterpret_cast<uint32_t*>(d)[i] = 0;
+    for (uint32_t b = lane; b < LZ_NB; b += 32) cnt[b] = 0;
+    for (uint32_t i = lane; i < L / 32u + 2u; i += 32) mark[i] = 0;
     __syncwarp();
 
-    // ---- bucket index of the positions with a full key (p + 2 < L) ----
+    // ---- positions with a full key (p + 2 < L), sorted by bucket ----
     const uint32_t np = L - 2u;
-    for (uint32_t p0 = 0; p0 < np; p0 += 32) {  // counts (one leader per distinct bucket)
-        const uint32_t p = p0 + lane;
-        const uint32_t h = p < np ? lz_hash(lz_key(d, p)) : LZ_NB + lane;
-        const uint32_t peers = __match_any_sync(GD_FULL_MASK, h);
-        if (p < np && (peers & ((1u << lane) - 1u)) == 0) cursor[h] += __popc(peers);
-        __syncwarp();
-    }
+    for (uint32_t p = lane; p < np; p += 32) atomicAdd(&cnt[lz_hash(lz_word(d, p))], 1u);
+    __syncwarp();
     {
         constexpr uint32_t PER = LZ_NB / 32u;
         uint32_t v[PER], sum = 0;
 #pragma unroll
         for (uint32_t i = 0; i < PER; ++i) {
-            v[i] = cursor[lane * PER + i];
+            v[i] = cnt[lane * PER + i];
             sum += v[i];
         }
         uint32_t run = warp_incl_scan(sum) - sum;
 #pragma unroll
-        for (uint32_t i = 0; i < PER; ++i) {
-            start[lane * PER + i] = (uint16_t)run;
+        for (uint32_t i = 0; i < PER; ++i) {  // where each bucket starts; its end once it is filled
+            end[lane * PER + i] = (uint16_t)run;
+            if (aged) oldest[lane * PER + i] = (uint16_t)run;
             run += v[i];
         }
-        if (lane == 31) start[LZ_NB] = (uint16_t)run;
     }
     __syncwarp();
-    for (uint32_t b = lane; b < LZ_NB; b += 32) cursor[b] = 0;
-    __syncwarp();
-    for (uint32_t p0 = 0; p0 < np; p0 += 32) {  // scatter, ascending inside each bucket
+    for (uint32_t p0 = 0; p0 < np; p0 += 32) {
         const uint32_t p = p0 + lane;
-        const uint32_t h = p < np ? lz_hash(lz_key(d, p)) : LZ_NB + lane;
+        const uint32_t h = p < np ? lz_hash(lz_word(d, p)) : LZ_NB + lane;
         const uint32_t peers = __match_any_sync(GD_FULL_MASK, h);
-        if (p < np) pos[start[h] + cursor[h] + __popc(peers & ((1u << lane) - 1u))] = (uint16_t)p;
+        uint32_t at = 0;
+        if (p < np) {
+            at = end[h] + __popc(peers & lt);
+            pos[at] = (uint16_t)p;
+        }
         __syncwarp();
-        if (p < np && (peers & ((1u << lane) - 1u)) == 0) cursor[h] += __popc(peers);
+        if (p < np && (peers >> lane) == 1u) end[h] = (uint16_t)(at + 1u);  // the last of its bucket here
         __syncwarp();
     }
-    for (uint32_t b = lane; b < LZ_NB; b += 32) cursor[b] = start[b];
+    // ---- mark the positions with a match: the same key 3 or more bytes back,
+    // inside the history (offset 0 of the column is never a source) ----
+    for (uint32_t x = lane; x < np; x += 32) {
+        const uint32_t p = pos[x], w = lz_word(d, p), h = lz_hash(w);
+        const uint32_t first = h ? end[h - 1u] : 0u, lo = p < LZ_HIST ? 1u : p - LZ_HIST + 1u;
+        for (uint32_t y = x; y > first;) {
+            const uint32_t c = pos[--y];
+            if (c < lo) break;
+            if (c + LZ_MINM <= p && ((lz_word(d, c) ^ w) & 0xffffffu) == 0) {
+                atomicOr(&mark[p >> 5], 1u << (p & 31u));
+                break;
+            }
+        }
+    }
     __syncwarp();
 
-    // ---- greedy token walk (warp-uniform), tokens written by lane 0 ----
-    DevSink o{reinterpret_cast<uint32_t*>(scratch + (uint64_t)col * cap), 0u, cap, 0u};
-    if (lane == 0) o.put(0);  // first flag byte
-    uint32_t flag_pos = 0, flags = 0, blocks = 0, cur = 0;
-    while (cur < L) {
-        const uint32_t hist_count = cur < LZ_HIST ? cur : LZ_HIST;
-        const uint32_t look = (L - cur) < LZ_LOOK ? (L - cur) : LZ_LOOK;
-        uint32_t best_len = 0, best_pos = 0;
-        if (look >= LZ_MINM && cur >= 3 && cur + 2 < L) {
-            const uint32_t lo = cur - hist_count + 1;  // the oldest history entry (offset 0 is never a source)
-            const uint32_t key = lz_key(d, cur), b = lz_hash(key);
-            const uint32_t end = start[b + 1];
-            uint32_t idx = cursor[b];
-            while (idx < end && pos[idx] < lo) ++idx;
+    // ---- greedy token walk (warp-uniform) ----
+    uint32_t* slot = reinterpret_cast<uint32_t*>(scratch + (uint64_t)col * cap);
+    uint32_t tok = 0, nt = 0;        // token `lane` of the queue (literal: 1 << 16 | byte), tokens queued
+    uint32_t on = 0, written = 0;    // bytes in out, words in the slot
+    bool over = false;
+    // write the queue's tokens, a flag byte before every 8; last: the stream
+    // ends, with a reserved flag byte if its last group is full
+    auto emit = [&](bool last) {
+        const uint32_t lits = __ballot_sync(GD_FULL_MASK, lane < nt && (tok >> 16) != 0);
+        const uint32_t size = lane < nt ? ((tok >> 16) ? 1u : 2u) + ((lane & 7u) == 0 ? 1u : 0u) : 0u;
+        const uint32_t inc = warp_incl_scan(size);
+        uint32_t at = on + inc - size;
+        if (size) {
+            if ((lane & 7u) == 0) out[at++] = (uint8_t)(lits >> lane);
+            out[at] = (uint8_t)tok;
+            if (!(tok >> 16)) out[at + 1] = (uint8_t)(tok >> 8);
+        }
+        on += __shfl_sync(GD_FULL_MASK, inc, 31);
+        if (last) {
+            if ((nt & 7u) == 0) {
+                if (lane == 0) out[on] = 0;
+                ++on;
+            }
+            if ((on & 3u) && (on & 3u) + lane < 4u) out[on + lane] = 0;
+        }
+        nt = 0;
+        __syncwarp();
+        if (on < LZ_OUT / 2u && !last) return;
+        const uint32_t nw = last ? (on + 3u) >> 2 : on >> 2;
+        over = over || 4u * (written + nw) > cap;
+        if (!over)
+            for (uint32_t w = lane; w < nw; w += 32) slot[written + w] = reinterpret_cast<const uint32_t*>(out)[w];
+        if (last) return;
+        written += nw;
+        on &= 3u;
+        uint8_t keep = 0;
+        if (lane < on) keep = out[4u * nw + lane];
+        __syncwarp();
+        if (lane < on) out[lane] = keep;
+        __syncwarp();
+    };
+    for (uint32_t cur = 0; cur < L;) {
+        // literals up to the next marked position
+        uint32_t m = mark[cur >> 5] >> (cur & 31u);
+        uint32_t lit = m ? (uint32_t)__ffs(m) - 1u : min(32u - (cur & 31u), L - cur);
+        while (lit) {
+            const uint32_t k = min(lit, 32u - nt);
+            if (lane - nt < k) tok = 0x10000u | d[cur + lane - nt];
+            nt += k;
+            cur += k;
+            lit -= k;
+            if (nt == 32) emit(false);
+        }
+        if (!m) continue;
+        // the longest match here
+        const uint32_t w = lz_word(d, cur), b = lz_hash(w), bend = end[b];
+        uint32_t idx = b ? end[b - 1u] : 0u;
+        if (aged) {
+            idx = oldest[b];
+            const uint32_t lo = cur < LZ_HIST ? 1u : cur - LZ_HIST + 1u;
+            while (idx < bend && pos[idx] < lo) ++idx;
             __syncwarp();
-            if (lane == 0) cursor[b] = (uint16_t)idx;
-            for (uint32_t base = idx; base < end; base += 32) {
-                const uint32_t j = base + lane;
-                const uint32_t p = j < end ? pos[j] : 0xffffu;
-                const bool valid = j < end && p + LZ_MINM <= cur;
-                uint32_t f = 0;
-                if (valid && lz_key(d, p) == key) {
-                    uint32_t lim = cur - p;
-                    lim = lim < look ? lim : look;
-                    lim = lim < LZ_MAXM ? lim : LZ_MAXM;
+            if (lane == 0) oldest[b] = (uint16_t)idx;
+        } else if (pos[idx] == 0) {
+            ++idx;
+        }
+        const uint32_t most = min(L - cur, LZ_MAXM);
+        uint32_t best_len = 0, best_pos = 0;
+        for (uint32_t base = idx; base < bend; base += 32) {
+            const uint32_t p = base + lane < bend ? pos[base + lane] : 0xffffu;
+            const bool valid = p + LZ_MINM <= cur;
+            uint32_t f = 0;
+            if (valid) {
+                const uint32_t x = lz_word(d, p) ^ w;
+                if ((x & 0xffffffu) == 0) {
+                    const uint32_t lim = min(cur - p, most);
                     f = 3;
-                    while (f < lim && d[p + f] == d[cur + f]) ++f;
+                    if (x == 0) {
+                        for (f = 4; f < lim; f += 4) {
+                            const uint32_t y = lz_word(d, p + f) ^ lz_word(d, cur + f);
+                            if (y) {
+                                f += (uint32_t)(__ffs(y) - 1) >> 3;
+                                break;
+                            }
+                        }
+                        f = min(f, lim);
+                    }
                 }
-                const uint32_t best = __reduce_max_sync(GD_FULL_MASK, f ? (f << 6) | (63u - lane) : 0u);
-                if ((best >> 6) > best_len) {
-                    best_len = best >> 6;
-                    best_pos = pos[base + 63u - (best & 63u)];
-                }
-                if (best_len >= LZ_MAXM || __any_sync(GD_FULL_MASK, !valid)) break;
             }
-        }
-        if (best_len < LZ_MINM) {
-            if (lane == 0) o.put(d[cur]);
-            flags |= 1u << blocks;
-            cur += 1;
-        } else {
-            const uint32_t v = ((cur - best_pos) << 5) | (best_len - LZ_MINM);
-            if (lane == 0) {
-                o.put((uint8_t)(v & 0xffu));
-                o.put((uint8_t)(v >> 8));
+            const uint32_t best = __reduce_max_sync(GD_FULL_MASK, f ? (f << 6) | (63u - lane) : 0u);
+            if ((best >> 6) > best_len) {
+                best_len = best >> 6;
+                best_pos = pos[base + 63u - (best & 63u)];
             }
-            cur += best_len;
+            if (best_len >= LZ_MAXM || __any_sync(GD_FULL_MASK, !valid)) break;
         }
-        if (++blocks == 8) {
-            if (lane == 0) {
-                o.set(flag_pos, (uint8_t)flags);
-                flag_pos = o.n;
-                o.put(0);  // the next flag byte is reserved even if no token follows
-            }
-            flags = 0;
-            blocks = 0;
-        }
+        if (lane == nt) tok = ((cur - best_pos) << 5) | (best_len - LZ_MINM);
+        ++nt;
+        cur += best_len;
+        if (nt == 32) emit(false);
     }
-    if (lane == 0) {
-        if (blocks != 0) o.set(flag_pos, (uint8_t)flags);
-        o.flush();
-        raw_len[col] = o.n <= cap ? o.n : 0xffffffffu;
-    }
+    emit(true);
+    if (lane == 0) raw_len[col] = over ? 0xffffffffu : 4u * written + on;
 }
 
 // A warp per chunk: slots are the columns by descending stream length (equal
