@@ -13,12 +13,14 @@
 // RLE v2: 8 adjacent lane streams per block, copied with fully used 32-byte
 // row sectors):
 //   * runs are closed form: lane i writes base + i*delta;
+//   * a header, a run's delta and a base of up to 4 bytes come from two
+//     funnel-shifted words (a longer base byte by byte);
 //   * a literal group is decoded 32 values at a time: the lanes load a
-//     128-byte window, ballot the varint terminators (bytes < 0x80), and lane
-//     j finds the j-th terminator (the mask quarter by comparison with the
-//     quarters' prefix counts, then one select), so every lane knows where
-//     its varint starts and ends and decodes it alone (32-bit values: one
-//     funnel-shifted word and a fifth byte, compacted with masks).
+//     128-byte window and ballot the varint terminators (bytes < 0x80); the
+//     lane at the j-th terminator stores its place for lane j (a select of the
+//     j-th set bit of the ballots by every lane took most of the step), so
+//     every lane knows where its varint starts and ends and decodes it alone
+//     (the first 4 bytes by one funnel-shifted word, compacted with masks).
 #pragma once
 #include "interleave.cuh"
 
@@ -35,6 +37,11 @@ __host__ __device__ constexpr uint32_t stream_cap(uint32_t nv, uint32_t eb) {
 // Shared-memory bytes reserved for a lane stream of at most `n` bytes.
 __host__ __device__ constexpr uint32_t lane_cap(uint32_t n) { return ((n + 15u) & ~15u) + 144u; }
 
+// The 7-bit groups of 4 varint bytes.
+__device__ __forceinline__ uint32_t low28(uint32_t v) {
+    return (v & 0x7fu) | ((v >> 1) & 0x3f80u) | ((v >> 2) & 0x1fc000u) | ((v >> 3) & 0xfe00000u);
+}
+
 // Decode one lane stream (sbuf[0..len), readable 144 bytes past len) of nv
 // elements of type T with the calling warp.  Lane stream t with wil = values
 // per lane slice: element e goes to outv[(e/wil)*32*wil + t*wil + e%wil] if
@@ -42,7 +49,9 @@ __host__ __device__ constexpr uint32_t lane_cap(uint32_t n) { return ((n + 15u) 
 template <typename T>
 static __device__ __noinline__ uint32_t lane_warp(const uint8_t* __restrict__ sbuf, uint32_t len, uint32_t nv, uint32_t t,
                                            uint32_t wil, T* __restrict__ outv, uint64_t want) {
+    __shared__ uint8_t s_ends[8][32];  // blocks have at most 8 warps
     const uint32_t lane = lane_id();
+    uint8_t* ends = s_ends[threadIdx.x >> 5];
     // wil a power of two (COMP_COL_LEN / sizeof(T) always is in the
     // reference's configurations): shifts instead of a division per value
     const bool pow2 = (wil & (wil - 1u)) == 0u;
@@ -60,36 +69,44 @@ static __device__ __noinline__ uint32_t lane_warp(const uint8_t* __restrict__ sb
         // ---- header: every lane parses it (shared-memory broadcast reads),
         // so nothing needs to be shuffled ----
         uint32_t kind = 0, cnt = 0, next = 0, e = ST_OK;
-        uint64_t base = 0, delta = 0;
-        {
-            uint32_t p = pos;
-            if (p >= len) {
-                e = ST_CORRUPT;
+        T base = 0, delta = 0;
+        if (pos >= len) {
+            e = ST_CORRUPT;
+        } else {
+            const uint32_t* w = reinterpret_cast<const uint32_t*>(sbuf + (pos & ~3u));
+            const uint32_t w1 = w[1], sh8 = 8u * (pos & 3u);
+            const uint32_t lo = __funnelshift_r(w[0], w1, sh8);  // the next 4 bytes
+            const uint32_t h = lo & 0xffu;
+            if (h & 0x80u) {
+                kind = 1;
+                cnt = 256u - h;
+                next = pos + 1;
             } else {
-                const uint32_t h = sbuf[p++];
-                if (h & 0x80u) {
-                    kind = 1;
-                    cnt = 256u - h;
-                } else if (p >= len) {
-                    e = ST_CORRUPT;
+                cnt = h + 3u;
+                delta = (T)(int64_t)(int8_t)(lo >> 8);
+                const uint32_t v = __funnelshift_r(lo, __funnelshift_r(w1, w[2], sh8), 16);  // the base's first 4
+                const uint32_t term = ~v & 0x80808080u;
+                if (term) {
+                    const uint32_t n = (__ffs(term) >> 3);  // bytes: 1 .. 4
+                    base = (T)low28(n < 4 ? v & ((1u << (8u * n)) - 1u) : v);
+                    next = pos + 2 + n;
+                    if (next > len) e = ST_CORRUPT;
                 } else {
-                    kind = 0;
-                    cnt = h + 3u;
-                    delta = (uint64_t)(int64_t)(int8_t)sbuf[p++];
-                    uint32_t sh = 0, b;
+                    uint32_t p = pos + 2, sh = 0, b;
+                    uint64_t x = 0;
                     do {
                         if (p >= len || sh > 63) {
                             e = ST_CORRUPT;
                             break;
                         }
                         b = sbuf[p++];
-                        base |= (uint64_t)(b & 0x7fu) << sh;
+                        x |= (uint64_t)(b & 0x7fu) << sh;
                         sh += 7;
                     } while (b & 0x80u);
-                    if (sizeof(T) == 4) base &= 0xffffffffull;
+                    base = (T)x;
+                    next = p;
                 }
             }
-            next = p;
         }
         if (e != ST_OK) {
             err = e;
@@ -100,7 +117,7 @@ static __device__ __noinline__ uint32_t lane_warp(const uint8_t* __restrict__ sb
             break;
         }
         if (kind == 0) {  // run: closed form (in T's width: the low bits of base + i*delta)
-            for (uint32_t i = lane; i < cnt; i += 32) put(g + i, (T)base + (T)i * (T)delta);
+            for (uint32_t i = lane; i < cnt; i += 32) put(g + i, base + (T)i * delta);
             g += cnt;
             pos = next;
             continue;
@@ -108,49 +125,38 @@ static __device__ __noinline__ uint32_t lane_warp(const uint8_t* __restrict__ sb
         // literal group: cnt varints starting at `next`
         uint32_t p = next, rem = cnt;
         while (rem) {
-            uint32_t m[4];
+            uint32_t m[4], nterm = 0;
 #pragma unroll
             for (int q = 0; q < 4; ++q) {
                 const uint32_t bpos = p + 32u * q + lane;
                 const bool term = (bpos < len) && !(sbuf[bpos] & 0x80u);
                 m[q] = __ballot_sync(GD_FULL_MASK, term);
+                const uint32_t rank = nterm + __popc(m[q] & ((1u << lane) - 1u));
+                if (term && rank < 32u) ends[rank] = (uint8_t)(32u * q + lane);
+                nterm += __popc(m[q]);
             }
-            const uint32_t c0 = __popc(m[0]), c01 = c0 + __popc(m[1]), c012 = c01 + __popc(m[2]);
-            const uint32_t nterm = c012 + __popc(m[3]);
             if (nterm == 0) {  // no varint ends within 128 bytes (or the stream ran out)
                 err = ST_CORRUPT;
                 break;
             }
             const uint32_t take = min(min(rem, nterm), 32u);
-            // lane j's varint ends at the j-th terminator: its 32-bit quarter
-            // of the mask by comparison, then one select within it
-            uint32_t end = 0;
-            if (lane < take) {
-                const uint32_t q = (lane >= c0) + (lane >= c01) + (lane >= c012);
-                const uint32_t mq = q == 0 ? m[0] : (q == 1 ? m[1] : (q == 2 ? m[2] : m[3]));
-                const uint32_t nq = lane - (q == 0 ? 0u : (q == 1 ? c0 : (q == 2 ? c01 : c012)));
-                end = 32u * q + __fns(mq, 0, (int)nq + 1);
-            }
+            __syncwarp();
+            const uint32_t end = lane < take ? ends[lane] : 0u;
             const uint32_t prev = __shfl_up_sync(GD_FULL_MASK, end, 1);  // the previous varint's last byte
             if (lane < take) {
                 const uint32_t beg = lane ? prev + 1 : 0;
-                uint64_t v = 0;
+                const uint32_t a = p + beg, n = end - beg + 1;
+                const uint32_t* wp = reinterpret_cast<const uint32_t*>(sbuf + (a & ~3u));
+                uint32_t lo = __funnelshift_r(wp[0], wp[1], 8u * (a & 3u));
+                if (n < 4) lo &= (1u << (8u * n)) - 1u;
+                T v = (T)low28(lo);
                 if constexpr (sizeof(T) == 4) {
-                    // a 32-bit value takes the varint's first 5 bytes: the
-                    // first 4 by one funnel-shifted word, 7 bits apiece
-                    const uint32_t a = p + beg, n = end - beg + 1;
-                    const uint32_t* wp = reinterpret_cast<const uint32_t*>(sbuf + (a & ~3u));
-                    uint32_t lo = __funnelshift_r(wp[0], wp[1], 8u * (a & 3u));
-                    if (n < 4) lo &= (1u << (8u * n)) - 1u;
-                    const uint32_t hi = n >= 5 ? (uint32_t)sbuf[a + 4] : 0u;
-                    v = (lo & 0x7fu) | ((lo >> 1) & 0x3f80u) | ((lo >> 2) & 0x1fc000u) | ((lo >> 3) & 0xfe00000u) |
-                        (hi << 28);
+                    // a 32-bit value takes the varint's first 5 bytes
+                    if (n >= 5) v |= (T)sbuf[a + 4] << 28;
                 } else {
-                    uint32_t sh = 0;
-                    for (uint32_t k = beg; k <= end; ++k, sh += 7)
-                        if (sh < 64) v |= (uint64_t)(sbuf[p + k] & 0x7fu) << sh;
+                    for (uint32_t k = 4; k < n && k < 10; ++k) v |= (T)(sbuf[a + k] & 0x7fu) << (7u * k);
                 }
-                put(g + lane, (T)v);
+                put(g + lane, v);
             }
             p += __shfl_sync(GD_FULL_MASK, end, take - 1) + 1;
             g += take;
