@@ -9,9 +9,9 @@ are compiled into libgd.so or sets a launch shape:
   brle     GD_TUNE_BRLE_BLOCKS_PER_SM     grid = value x SMs
   rlev1    GD_TUNE_RLEV1_LANES_PER_BLOCK  lane streams (warps) per block
   rlev2    GD_TUNE_RLEV2_LANES_PER_BLOCK  lane streams (warps) per block
-  lzss     GD_TUNE_LZSS_WARPS_PER_BLOCK   0: a warp per chunk, a lane per column, output in rounds
-                                          (1 chunk per block), 4: the same, 4 per block; 512 / 256:
-                                          16 / 8 lanes per column, 1: a lane per column (these stage
+  lzss     GD_TUNE_LZSS_WARPS_PER_BLOCK   0: a warp per column, a lane per token; 4: a warp per chunk, a
+                                          lane per column, output in rounds, 4 chunks per block; 512 /
+                                          256: 16 / 8 lanes per column, 1: a lane per column (these stage
                                           the whole chunk in shared memory)
 
 For the batched decoder the tuned quantity is its blocks per SM (8 warps each),

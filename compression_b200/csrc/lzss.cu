@@ -1,6 +1,7 @@
 // lzss.cu -- LZSS (32-column interleaved container) decoder for sm_100a.
 // The decoders are in lzss.cuh; GD_TUNE_LZSS_WARPS_PER_BLOCK selects one.
 #include "lzss.cuh"
+#include "lzss_follow.cuh"
 
 namespace gd {
 namespace lzss {
@@ -111,6 +112,23 @@ extern "C" gd_status_t gd_lzss_decode(const uint8_t* d_data, const uint64_t* d_b
                              cudaSharedmemCarveoutMaxShared);
         decode_staged_kernel<<<n_chunks, 32, staged, (cudaStream_t)stream>>>(d_data, d_blk_off, d_col_len, d_col_map,
                                                                             n_chunks, chunk_size, d_out, d_status);
+        return cudaGetLastError() == cudaSuccess ? GD_OK : GD_ERR_CUDA;
+    }
+    // columns of up to 4 KiB, 16-byte row stores: a block per 8 columns (5 an
+    // SM at 2 KiB), or per 4 where 8 columns' workspaces leave room for two
+    // blocks on an SM only (128 KiB chunks: 1.63 ms for 256 MiB)
+    if (k == 0 && chunk_size / 32 <= FMAXL && (reinterpret_cast<uintptr_t>(d_out) & 15u) == 0) {
+        const uint32_t L = (uint32_t)(chunk_size / 32);
+        cudaStream_t s = (cudaStream_t)stream;
+        if (d_status && cudaMemsetAsync(d_status, 0, 4ull * n_chunks, s) != cudaSuccess) return GD_ERR_CUDA;
+        auto go = [&](auto kern, uint32_t cols) {
+            const uint32_t smem = cols * follow_col_smem(L);
+            cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+            kern<<<n_chunks * (32u / cols), cols * 32, smem, s>>>(d_data, d_blk_off, d_col_len, d_col_map, L, d_out,
+                                                                 d_status);
+        };
+        if (8u * follow_col_smem(L) <= 45u * 1024u) go(decode_follow_kernel<8>, 8);
+        else go(decode_follow_kernel<4>, 4);
         return cudaGetLastError() == cudaSuccess ? GD_OK : GD_ERR_CUDA;
     }
     // group decoder (any chunk size): one chunk per 32-thread block with

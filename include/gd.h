@@ -294,12 +294,13 @@ typedef enum gd_tune_key {
     GD_TUNE_RLEV1_LANES_PER_BLOCK = 2, /* 0/8: 8 lane streams per block; 4: 4 */
     GD_TUNE_RLEV2_LANES_PER_BLOCK = 3, /* 0: 8 lane streams per block (4 if 8 do not fit in shared
                                           memory); 8: 8; 4: 4 */
-    GD_TUNE_LZSS_WARPS_PER_BLOCK = 4,  /* 0: one chunk per 32-thread block, one lane per column, a
-                                          flag group per lane and step, output in 320-byte rounds
-                                          per column (any chunk size); 4: the same with four chunks
-                                          per block and 256-byte rounds (the batch decoder's shape);
-                                          512 / 256: one chunk per block of 512 / 256 threads, 16 / 8
-                                          lanes per column, output staged in shared memory; 1: one
+    GD_TUNE_LZSS_WARPS_PER_BLOCK = 4,  /* 0: a warp per column, 8 or 4 columns per block, a lane per token
+                                          (chunks up to 128 KiB; longer ones, and output not 16-byte
+                                          aligned: one chunk per 32-thread block, one lane per column, a
+                                          flag group per lane and step, output in 320-byte rounds per
+                                          column); 4: that with four chunks per block and 256-byte
+                                          rounds; 512 / 256: one chunk per block of 512 / 256 threads,
+                                          16 / 8 lanes per column, output staged in shared memory; 1: one
                                           chunk per warp, one lane per column, output staged */
     GD_TUNE_INFLATE_PAIR_SPIN = 5,     /* polls of a decoder/writer hand-off wait before the stream
                                           gives up with GD_ERR_TIMEOUT (0: 2^25, about a second) */
