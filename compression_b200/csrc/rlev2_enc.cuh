@@ -325,16 +325,18 @@ __global__ void __launch_bounds__(V2_WPB * 32) rlev2_encode_kernel(const uint8_t
     int64_t stale = 0;
     // value k of the lane is chunk value (k / ru) * 32 * ru + t * ru + k % ru
     // (encoder_trans.h:40-108); values past the input are zero
+    auto fetch = [&](uint32_t k) -> int64_t {
+        if (k >= n) return 0;
+        const uint32_t q = k / read_unit;
+        const uint64_t at = (uint64_t)q * 32u * read_unit + (uint64_t)t * read_unit + (k - q * read_unit);
+        return at < avail ? __ldg(base + at) : 0;
+    };
+    int64_t ahead = fetch(lane);  // values loaded .. loaded + 31, on their way
     for (uint32_t i = 0; i < n;) {
         while (loaded < n && loaded < i + 128u) {
-            const uint32_t k = loaded + lane;
-            int64_t v = 0;
-            if (k < n) {
-                const uint32_t q = k / read_unit;
-                const uint64_t at = (uint64_t)q * 32u * read_unit + (uint64_t)t * read_unit + (k - q * read_unit);
-                if (at < avail) v = __ldg(base + at);
-            }
-            S.ring[k & 255u] = v;
+            const int64_t v = ahead;
+            ahead = fetch(loaded + 32u + lane);
+            S.ring[(loaded + lane) & 255u] = v;
             const int64_t up = __shfl_down_sync(GD_FULL_MASK, v, 1);
             const uint32_t e = __ballot_sync(GD_FULL_MASK, lane < 31 && up == v);
             if (lane == 0) {
