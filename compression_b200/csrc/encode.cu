@@ -192,9 +192,10 @@ __global__ void __launch_bounds__(LZ_WPB * 32) lzss_column_kernel(const uint8_t*
     for (uint32_t i = lane; i < L / 32u + 2u; i += 32) mark[i] = 0;
     __syncwarp();
 
-    // ---- positions with a full key (p + 2 < L), sorted by bucket ----
+    // ---- positions with a full key (p + 2 < L), sorted by bucket; not the
+    // first, which is never a source ----
     const uint32_t np = L - 2u;
-    for (uint32_t p = lane; p < np; p += 32) atomicAdd(&cnt[lz_hash(lz_word(d, p))], 1u);
+    for (uint32_t p = 1u + lane; p < np; p += 32) atomicAdd(&cnt[lz_hash(lz_word(d, p))], 1u);
     __syncwarp();
     {
         constexpr uint32_t PER = LZ_NB / 32u;
@@ -213,7 +214,7 @@ __global__ void __launch_bounds__(LZ_WPB * 32) lzss_column_kernel(const uint8_t*
         }
     }
     __syncwarp();
-    for (uint32_t p0 = 0; p0 < np; p0 += 32) {
+    for (uint32_t p0 = 1; p0 < np; p0 += 32) {
         const uint32_t p = p0 + lane;
         const uint32_t h = p < np ? lz_hash(lz_word(d, p)) : LZ_NB + lane;
         const uint32_t peers = __match_any_sync(GD_FULL_MASK, h);
@@ -227,10 +228,10 @@ __global__ void __launch_bounds__(LZ_WPB * 32) lzss_column_kernel(const uint8_t*
         __syncwarp();
     }
     // ---- mark the positions with a match: the same key 3 or more bytes back,
-    // inside the history (offset 0 of the column is never a source) ----
-    for (uint32_t x = lane; x < np; x += 32) {
+    // inside the history ----
+    for (uint32_t x = lane; x + 1u < np; x += 32) {
         const uint32_t p = pos[x], w = lz_word(d, p), h = lz_hash(w);
-        const uint32_t first = h ? end[h - 1u] : 0u, lo = p < LZ_HIST ? 1u : p - LZ_HIST + 1u;
+        const uint32_t first = h ? end[h - 1u] : 0u, lo = p < LZ_HIST ? 0u : p - LZ_HIST + 1u;
         for (uint32_t y = x; y > first;) {
             const uint32_t c = pos[--y];
             if (c < lo) break;
@@ -301,14 +302,12 @@ __global__ void __launch_bounds__(LZ_WPB * 32) lzss_column_kernel(const uint8_t*
         uint32_t idx = b ? end[b - 1u] : 0u;
         if (aged) {
             idx = oldest[b];
-            const uint32_t lo = cur < LZ_HIST ? 1u : cur - LZ_HIST + 1u;
+            const uint32_t lo = cur < LZ_HIST ? 0u : cur - LZ_HIST + 1u;
             while (idx < bend && pos[idx] < lo) ++idx;
             __syncwarp();
             if (lane == 0) oldest[b] = (uint16_t)idx;
-        } else if (pos[idx] == 0) {
-            ++idx;
         }
-        const uint32_t most = min(L - cur, LZ_MAXM);
+        const uint32_t most = min(L - cur, LZ_MAXM), w4 = lz_word(d, cur + 4u);
         uint32_t best_len = 0, best_pos = 0;
         for (uint32_t base = idx; base < bend; base += 32) {
             const uint32_t p = base + lane < bend ? pos[base + lane] : 0xffffu;
@@ -320,21 +319,25 @@ __global__ void __launch_bounds__(LZ_WPB * 32) lzss_column_kernel(const uint8_t*
                     const uint32_t lim = min(cur - p, most);
                     f = 3;
                     if (x == 0) {
-                        for (f = 4; f < lim; f += 4) {
-                            const uint32_t y = lz_word(d, p + f) ^ lz_word(d, cur + f);
-                            if (y) {
-                                f += (uint32_t)(__ffs(y) - 1) >> 3;
-                                break;
+                        const uint32_t y4 = lz_word(d, p + 4u) ^ w4;
+                        f = y4 ? 4u + ((uint32_t)(__ffs(y4) - 1) >> 3) : 8u;
+                        if (!y4)
+                            for (; f < lim; f += 4) {
+                                const uint32_t y = lz_word(d, p + f) ^ lz_word(d, cur + f);
+                                if (y) {
+                                    f += (uint32_t)(__ffs(y) - 1) >> 3;
+                                    break;
+                                }
                             }
-                        }
                         f = min(f, lim);
                     }
                 }
             }
             const uint32_t best = __reduce_max_sync(GD_FULL_MASK, f ? (f << 6) | (63u - lane) : 0u);
+            const uint32_t from = __shfl_sync(GD_FULL_MASK, p, 63 - (int)(best & 63u));
             if ((best >> 6) > best_len) {
                 best_len = best >> 6;
-                best_pos = pos[base + 63u - (best & 63u)];
+                best_pos = from;
             }
             if (best_len >= LZ_MAXM || __any_sync(GD_FULL_MASK, !valid)) break;
         }
