@@ -392,6 +392,10 @@ def _sub(cont, a, b):
     """Chunks [a, b) of an oracle container as a container of their own."""
     import oracle
     m, cs = cont.meta, cont.chunk_size
+    if cont.codec == "brle":
+        p = m["ptr"]
+        return oracle.Container("brle", cont.data[int(p[a]):int(p[b])], min(cont.n_out, b * cs) - a * cs, b - a, cs,
+                                {"ptr": (p[a:b + 1] - p[a]).astype(np.uint64)}, {})
     if cont.codec in ("rlev1", "rlev2", "lzss"):
         bo = m["blk_off"]
         meta = {"blk_off": (bo[a:b + 1] - bo[a]).astype(np.uint64), "col_len": m["col_len"][32 * a:32 * b]}
