@@ -18,6 +18,7 @@ Reference interfaces mirrored (ZaidQureshi/compression):
 from __future__ import annotations
 
 import ctypes as C
+import threading
 from dataclasses import dataclass, field
 
 import numpy as np
@@ -507,6 +508,36 @@ class DeviceJob:
         return self.d_out[: self.enc.n_out].cpu().numpy()
 
 
+class _Lent:
+    """An output buffer of the library (page-locked, from its cache) that a
+    result array uses in place; gd_free takes it back when the array and its
+    views are gone.  Copying a result out of page-locked memory took as long
+    as the rest of a 3 MB call (0.18 of 0.36 ms).  Bounded, because page-locked
+    memory is scarce: results beyond the limits are copied."""
+    MAX_BUFFERS, MAX_BYTES = 4, 256 << 20
+    _lock = threading.RLock()  # __del__ may run inside take()
+    _buffers = _bytes = 0
+
+    @classmethod
+    def take(cls, ptr: int, n: int):
+        """The array over n bytes at ptr, or None if too much is lent already."""
+        with cls._lock:
+            if cls._buffers >= cls.MAX_BUFFERS or cls._bytes + n > cls.MAX_BYTES:
+                return None
+            cls._buffers += 1
+            cls._bytes += n
+        o = cls()
+        o.ptr, o.n, o.free = ptr, n, lib().gd_free
+        o.__array_interface__ = {"data": (ptr, False), "shape": (n,), "typestr": "|u1", "version": 3}
+        return np.asarray(o)
+
+    def __del__(self):
+        with _Lent._lock:
+            _Lent._buffers -= 1
+            _Lent._bytes -= self.n
+        self.free(C.c_void_p(self.ptr))
+
+
 _PINNED_KEEP: list = []  # pinned tensors backing the numpy views below
 
 
@@ -590,6 +621,10 @@ def decode_host(enc: Encoded, keep: bool = True) -> np.ndarray:
         raise ValueError(enc.codec)
     check(rc, f"{enc.codec} host decompress")
     res = None
+    if keep and n.value:
+        res = _Lent.take(out.value, n.value)
+        if res is not None:
+            return res
     if keep:
         res = np.ctypeslib.as_array(C.cast(out, C.POINTER(C.c_uint8)), shape=(n.value,)).copy() if n.value else \
             np.empty(0, np.uint8)

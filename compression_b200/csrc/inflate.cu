@@ -147,12 +147,9 @@ template <int NW, uint32_t WIN, uint32_t NC, uint32_t TMAX, int BPS, class Chunk
 gd_status_t launch_block(const Chunks& ch, uint32_t n, int zlib_hdr, const uint32_t* order, cudaStream_t s) {
     using SmemT = gd::inflb::Smem<NW, WIN, NC, TMAX>;
     auto kern = gd::inflb::inflate_block_kernel<Chunks, SmemT, BPS>;
-    static bool attr_set = false;  // benign race: the attribute call is idempotent
-    if (!attr_set) {
-        if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, sizeof(SmemT)) != cudaSuccess)
-            return GD_ERR_CUDA;
-        attr_set = true;
-    }
+    // per device, so set at every call
+    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, sizeof(SmemT)) != cudaSuccess)
+        return GD_ERR_CUDA;
     kern<<<n, SmemT::NT, sizeof(SmemT), s>>>(ch, zlib_hdr, order);
     return cudaGetLastError() == cudaSuccess ? GD_OK : GD_ERR_CUDA;
 }
