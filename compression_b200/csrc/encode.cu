@@ -121,31 +121,43 @@ inline dim3 interleave_grid(uint64_t n_chunks, uint64_t lane_cap) {
 // greedy writer takes at every position the oldest of the longest matches in
 // the 2048-byte history (find_match, lzss_gpu2.h:70-108), so a position's
 // match depends only on the position.  A warp per column:
-//   - stages the column in shared memory and sorts its positions by a hash of
-//     their 3-byte keys, ascending inside a bucket;
-//   - marks the positions that have a match, a lane per sorted position
-//     looking back in its bucket for its key (usually the entry before);
-//   - walks the tokens: literals up to the next marked position in one step,
-//     and there the bucket's candidates 32 at a time, oldest first (one lane
-//     per candidate, compared 4 bytes at a time, the longest with the oldest
-//     winning ties), stopping at a 34-byte match;
-//   - queues tokens a lane each and writes 32 (four flag groups) together.
-// Searching at every token, literals too (64% of the benchmark's), and writing
-// each token from one lane took 88 warp instructions a token and 5.66 ms for
-// 64 MiB.  (Finding every position's match with a lane per position was 2.4x
-// slower still: the candidate lists are long, and serial per lane.)
+//   - stages the column in shared memory and counts its positions by a hash of
+//     their 3-byte keys, so that each bucket has its place;
+//   - takes 32 positions at a time, a lane each: puts them into their buckets
+//     (ascending inside each), finds the matches of all 32, a lane per pair of
+//     a position and an older one of its bucket (compared 4 bytes at a time;
+//     the longest match, then the oldest, is the largest of 16 bits), and then
+//     the positions that the greedy walk visits, by doubling its jumps;
+//   - where the 32 positions have more than LZ_PAIRS such pairs (long runs, few
+//     distinct keys), walks them token by token instead, the candidates 32 at a
+//     time from the oldest on, stopping at a 34-byte match;
+//   - writes their tokens, a lane each, to a small buffer that leaves in words;
+//     the open group's flag byte is rewritten until its 8 tokens are there.
+// Bound by issue (66% of the slots at 24 warps per SM, set by shared memory).
+// 64 MiB of Markov text with copies (a column: 383 matches, 618 literals,
+// 7700 pairs in most, 45,000 in one of a hundred): 2.2 ms, 45,500 warp
+// instructions a column, of which the pairs take 17,000 (62 for each 32), the
+// windows that go token by token 7000, and the rest of a window about 200.
+// Literals queued up to the next position with a match, then its candidates 32
+// at a time (6.6 are in a bucket), took 3.2 ms; searching at every token 5.66.
+// LZ_PAIRS: 256 2.15, 512 2.17, no limit 3.4 ms (columns of many pairs last
+// longest).  320 buckets, for 7 blocks per SM, 2.22 ms; 1024, for 5, 2.40; the
+// next pairs fetched ahead 2.18 ms.
+// (Finding every position's match with a lane per position was slower still:
+// the candidate lists differ in length, and are serial per lane.)
 
 constexpr uint32_t LZ_WPB = 4;      // columns (warps) per block
 constexpr uint32_t LZ_NB = 512;     // hash buckets of 3-byte keys
 constexpr uint32_t LZ_HIST = 2048, LZ_MAXM = 34, LZ_MINM = 3;
-constexpr uint32_t LZ_OUT = 256;    // output bytes held back: less than 128, and the next 32 tokens
+constexpr uint32_t LZ_OUT = 256;    // output bytes held back: less than 128, and the next 32 tokens' (37 at most)
+constexpr uint32_t LZ_PAIRS = 256;  // pairs of 32 positions found at once
 
 __host__ __device__ constexpr uint32_t a16(uint32_t x) { return (x + 15u) & ~15u; }
-// column bytes (+64 zero pad) | positions by bucket, also the counts before them | bucket ends | marks | output |
-// oldest candidates by bucket, where the column is longer than the history
+// column bytes (+64 zero pad) | positions by bucket, also the counts before them | bucket ends | bucket starts (the
+// oldest in the history) | a word per lane | output
 __host__ __device__ constexpr uint32_t lz_pos_bytes(uint32_t L) { return a16(2u * L > 4u * LZ_NB ? 2u * L : 4u * LZ_NB); }
 __host__ __device__ constexpr uint32_t lz_warp_smem(uint32_t L) {
-    return a16(L + 64u) + lz_pos_bytes(L) + a16(2u * LZ_NB) + a16(L / 8u + 8u) + LZ_OUT + (L > LZ_HIST ? a16(2u * LZ_NB) : 0u);
+    return a16(L + 64u) + lz_pos_bytes(L) + 4u * LZ_NB + 128u + LZ_OUT;
 }
 // the 4 bytes at p
 __device__ __forceinline__ uint32_t lz_word(const uint8_t* d, uint32_t p) {
@@ -168,9 +180,9 @@ __global__ void __launch_bounds__(LZ_WPB * 32) lzss_column_kernel(const uint8_t*
     uint16_t* pos = reinterpret_cast<uint16_t*>(d + a16(L + 64u));
     uint32_t* cnt = reinterpret_cast<uint32_t*>(pos);
     uint16_t* end = reinterpret_cast<uint16_t*>(reinterpret_cast<uint8_t*>(pos) + lz_pos_bytes(L));
-    uint32_t* mark = reinterpret_cast<uint32_t*>(reinterpret_cast<uint8_t*>(end) + a16(2u * LZ_NB));
-    uint8_t* out = reinterpret_cast<uint8_t*>(mark) + a16(L / 8u + 8u);
-    uint16_t* oldest = reinterpret_cast<uint16_t*>(out + LZ_OUT);
+    uint16_t* start = end + LZ_NB;
+    uint32_t* area = reinterpret_cast<uint32_t*>(start + LZ_NB);
+    uint8_t* out = reinterpret_cast<uint8_t*>(area + 32);
     const bool aged = L > LZ_HIST;  // candidates can leave the history
 
     // ---- the column: word k = chunk bytes [128k + 4q, +4); zero past the input ----
@@ -189,11 +201,10 @@ __global__ void __launch_bounds__(LZ_WPB * 32) lzss_column_kernel(const uint8_t*
     }
     for (uint32_t i = L / 4u + lane; i < L / 4u + 16u; i += 32) reinterpret_cast<uint32_t*>(d)[i] = 0;
     for (uint32_t b = lane; b < LZ_NB; b += 32) cnt[b] = 0;
-    for (uint32_t i = lane; i < L / 32u + 2u; i += 32) mark[i] = 0;
     __syncwarp();
 
-    // ---- positions with a full key (p + 2 < L), sorted by bucket; not the
-    // first, which is never a source ----
+    // ---- where each bucket of the positions with a full key (p + 2 < L)
+    // starts; not the first, which is never a source ----
     const uint32_t np = L - 2u;
     for (uint32_t p = 1u + lane; p < np; p += 32) atomicAdd(&cnt[lz_hash(lz_word(d, p))], 1u);
     __syncwarp();
@@ -207,146 +218,170 @@ __global__ void __launch_bounds__(LZ_WPB * 32) lzss_column_kernel(const uint8_t*
         }
         uint32_t run = warp_incl_scan(sum) - sum;
 #pragma unroll
-        for (uint32_t i = 0; i < PER; ++i) {  // where each bucket starts; its end once it is filled
-            end[lane * PER + i] = (uint16_t)run;
-            if (aged) oldest[lane * PER + i] = (uint16_t)run;
+        for (uint32_t i = 0; i < PER; ++i) {
+            start[lane * PER + i] = end[lane * PER + i] = (uint16_t)run;
             run += v[i];
         }
     }
     __syncwarp();
-    for (uint32_t p0 = 1; p0 < np; p0 += 32) {
-        const uint32_t p = p0 + lane;
-        const uint32_t h = p < np ? lz_hash(lz_word(d, p)) : LZ_NB + lane;
-        const uint32_t peers = __match_any_sync(GD_FULL_MASK, h);
-        uint32_t at = 0;
-        if (p < np) {
-            at = end[h] + __popc(peers & lt);
-            pos[at] = (uint16_t)p;
-        }
-        __syncwarp();
-        if (p < np && (peers >> lane) == 1u) end[h] = (uint16_t)(at + 1u);  // the last of its bucket here
-        __syncwarp();
-    }
-    // ---- mark the positions with a match: the same key 3 or more bytes back,
-    // inside the history ----
-    for (uint32_t x = lane; x + 1u < np; x += 32) {
-        const uint32_t p = pos[x], w = lz_word(d, p), h = lz_hash(w);
-        const uint32_t first = h ? end[h - 1u] : 0u, lo = p < LZ_HIST ? 0u : p - LZ_HIST + 1u;
-        for (uint32_t y = x; y > first;) {
-            const uint32_t c = pos[--y];
-            if (c < lo) break;
-            if (c + LZ_MINM <= p && ((lz_word(d, c) ^ w) & 0xffffffu) == 0) {
-                atomicOr(&mark[p >> 5], 1u << (p & 31u));
-                break;
-            }
-        }
-    }
-    __syncwarp();
 
-    // ---- greedy token walk (warp-uniform) ----
     uint32_t* slot = reinterpret_cast<uint32_t*>(scratch + (uint64_t)col * cap);
-    uint32_t tok = 0, nt = 0;        // token `lane` of the queue (literal: 1 << 16 | byte), tokens queued
-    uint32_t on = 0, written = 0;    // bytes in out, words in the slot
+    uint32_t on = 0, written = 0;              // bytes in out, words in the slot
+    uint32_t nt = 0, flag_at = 0, flag = 0;    // tokens in the open group (0: none is), its flag byte's place, and bits
     bool over = false;
-    // write the queue's tokens, a flag byte before every 8; last: the stream
-    // ends, with a reserved flag byte if its last group is full
-    auto emit = [&](bool last) {
-        const uint32_t lits = __ballot_sync(GD_FULL_MASK, lane < nt && (tok >> 16) != 0);
-        const uint32_t size = lane < nt ? ((tok >> 16) ? 1u : 2u) + ((lane & 7u) == 0 ? 1u : 0u) : 0u;
-        const uint32_t inc = warp_incl_scan(size);
-        uint32_t at = on + inc - size;
-        if (size) {
-            if ((lane & 7u) == 0) out[at++] = (uint8_t)(lits >> lane);
-            out[at] = (uint8_t)tok;
-            if (!(tok >> 16)) out[at + 1] = (uint8_t)(tok >> 8);
-        }
-        on += __shfl_sync(GD_FULL_MASK, inc, 31);
-        if (last) {
-            if ((nt & 7u) == 0) {
-                if (lane == 0) out[on] = 0;
-                ++on;
-            }
-            if ((on & 3u) && (on & 3u) + lane < 4u) out[on + lane] = 0;
-        }
-        nt = 0;
-        __syncwarp();
-        if (on < LZ_OUT / 2u && !last) return;
-        const uint32_t nw = last ? (on + 3u) >> 2 : on >> 2;
-        over = over || 4u * (written + nw) > cap;
-        if (!over)
-            for (uint32_t w = lane; w < nw; w += 32) slot[written + w] = reinterpret_cast<const uint32_t*>(out)[w];
-        if (last) return;
-        written += nw;
-        on &= 3u;
-        uint8_t keep = 0;
-        if (lane < on) keep = out[4u * nw + lane];
-        __syncwarp();
-        if (lane < on) out[lane] = keep;
-        __syncwarp();
-    };
-    for (uint32_t cur = 0; cur < L;) {
-        // literals up to the next marked position
-        uint32_t m = mark[cur >> 5] >> (cur & 31u);
-        uint32_t lit = m ? (uint32_t)__ffs(m) - 1u : min(32u - (cur & 31u), L - cur);
-        while (lit) {
-            const uint32_t k = min(lit, 32u - nt);
-            if (lane - nt < k) tok = 0x10000u | d[cur + lane - nt];
-            nt += k;
-            cur += k;
-            lit -= k;
-            if (nt == 32) emit(false);
-        }
-        if (!m) continue;
-        // the longest match here
-        const uint32_t w = lz_word(d, cur), b = lz_hash(w), bend = end[b];
-        uint32_t idx = b ? end[b - 1u] : 0u;
-        if (aged) {
-            idx = oldest[b];
-            const uint32_t lo = cur < LZ_HIST ? 0u : cur - LZ_HIST + 1u;
-            while (idx < bend && pos[idx] < lo) ++idx;
-            __syncwarp();
-            if (lane == 0) oldest[b] = (uint16_t)idx;
-        }
-        const uint32_t most = min(L - cur, LZ_MAXM), w4 = lz_word(d, cur + 4u);
-        uint32_t best_len = 0, best_pos = 0;
-        for (uint32_t base = idx; base < bend; base += 32) {
-            const uint32_t p = base + lane < bend ? pos[base + lane] : 0xffffu;
-            const bool valid = p + LZ_MINM <= cur;
-            uint32_t f = 0;
-            if (valid) {
-                const uint32_t x = lz_word(d, p) ^ w;
-                if ((x & 0xffffffu) == 0) {
-                    const uint32_t lim = min(cur - p, most);
-                    f = 3;
-                    if (x == 0) {
-                        const uint32_t y4 = lz_word(d, p + 4u) ^ w4;
-                        f = y4 ? 4u + ((uint32_t)(__ffs(y4) - 1) >> 3) : 8u;
-                        if (!y4)
-                            for (; f < lim; f += 4) {
-                                const uint32_t y = lz_word(d, p + f) ^ lz_word(d, cur + f);
-                                if (y) {
-                                    f += (uint32_t)(__ffs(y) - 1) >> 3;
-                                    break;
-                                }
-                            }
-                        f = min(f, lim);
-                    }
+    // length of the match of the candidate c with the bytes at p (w, w4: the
+    // words at p and p + 4), 0 if there is none
+    auto match = [&](uint32_t c, uint32_t p, uint32_t w, uint32_t w4) -> uint32_t {
+        const uint32_t* q = reinterpret_cast<const uint32_t*>(d) + (c >> 2);
+        const uint32_t a0 = q[0], a1 = q[1], a2 = q[2], sh = 8u * (c & 3u);
+        const uint32_t x = __funnelshift_r(a0, a1, sh) ^ w, y = __funnelshift_r(a1, a2, sh) ^ w4;
+        uint32_t f = (uint32_t)(x ? __clz(__brev(x)) : 32 + __clz(__brev(y))) >> 3;
+        const uint32_t off = p - c, lim = min(off, min(L - p, LZ_MAXM));
+        if (off - LZ_MINM >= LZ_HIST - LZ_MINM) return 0;  // too near, or too old
+        if (f == 8)
+            for (; f < lim; f += 4) {
+                const uint32_t z = lz_word(d, c + f) ^ lz_word(d, p + f);
+                if (z) {
+                    f += (uint32_t)(__ffs(z) - 1) >> 3;
+                    break;
                 }
             }
-            const uint32_t best = __reduce_max_sync(GD_FULL_MASK, f ? (f << 6) | (63u - lane) : 0u);
-            const uint32_t from = __shfl_sync(GD_FULL_MASK, p, 63 - (int)(best & 63u));
-            if ((best >> 6) > best_len) {
-                best_len = best >> 6;
-                best_pos = from;
-            }
-            if (best_len >= LZ_MAXM || __any_sync(GD_FULL_MASK, !valid)) break;
+        f = min(f, lim);
+        return f < LZ_MINM ? 0u : f;
+    };
+    uint32_t cur = 0;  // the next token's position
+    for (uint32_t w0 = 0; w0 < L; w0 += 32) {
+        // ---- the next 32 positions into their buckets ----
+        const uint32_t p = w0 + lane, w = lz_word(d, p);
+        const bool keyed = p >= 1u && p < np;
+        const uint32_t h = keyed ? lz_hash(w) : LZ_NB + lane;
+        const uint32_t peers = __match_any_sync(GD_FULL_MASK, h);
+        uint32_t at = 0, first = 0;
+        if (keyed) {
+            at = end[h] + __popc(peers & lt);
+            pos[at] = (uint16_t)p;
+            first = start[h];
+            if (aged)
+                while (first < at && pos[first] + LZ_HIST <= w0) ++first;  // too old for all 32, and those after
         }
-        if (lane == nt) tok = ((cur - best_pos) << 5) | (best_len - LZ_MINM);
-        ++nt;
-        cur += best_len;
-        if (nt == 32) emit(false);
+        __syncwarp();
+        if (keyed && (peers >> lane) == 1u) {  // the last of its bucket here
+            end[h] = (uint16_t)(at + 1u);
+            if (aged) start[h] = (uint16_t)first;
+        }
+        __syncwarp();
+        if (cur >= w0 + 32u) continue;
+        // ---- matches: a lane per (position, older position of its bucket) ----
+        const uint32_t n = keyed && p >= cur ? at - first : 0u;
+        const uint32_t w4 = lz_word(d, p + 4u);
+        const uint32_t inc = warp_incl_scan(n), total = __shfl_sync(GD_FULL_MASK, inc, 31);
+        uint32_t len = 1, next = w & 0xffu;  // this position's token: a byte, or a match's two
+        uint32_t reach = cur < L ? 1u << (cur - w0) : 0u;  // positions where a token starts
+        if (total <= LZ_PAIRS) {
+            // a word per list: its position, and where it lies in pos, less the pairs before it
+            const uint32_t excl = inc - n, has = __ballot_sync(GD_FULL_MASK, n != 0);
+            if (n) area[__popc(has & lt)] = (first - excl) << 5 | lane;
+            __syncwarp();
+            const uint32_t list = area[lane];
+            __syncwarp();
+            area[lane] = 0;
+            __syncwarp();
+            uint32_t before = 0;  // lists that start before the step
+            for (uint32_t t = 0; t < total; t += 32) {
+                const uint32_t s =
+                    __reduce_or_sync(GD_FULL_MASK, n && excl - t < 32u ? 1u << (excl - t) : 0u);  // lists that start here
+                const uint32_t mine = __shfl_sync(GD_FULL_MASK, list, (int)(before + __popc(s & (lt << 1 | 1u)) - 1u));
+                const uint32_t ow = __shfl_sync(GD_FULL_MASK, w, (int)(mine & 31u));
+                const uint32_t ow4 = __shfl_sync(GD_FULL_MASK, w4, (int)(mine & 31u));
+                before += __popc(s);
+                if (t + lane < total) {
+                    const uint32_t at0 = (uint32_t)((int32_t)mine >> 5) + t + lane, o = mine & 31u;
+                    const uint32_t c = pos[at0], f = match(c, w0 + o, ow, ow4);
+                    if (f) atomicMax(&area[o], (f - LZ_MINM) << 11 | (w0 + o - c));
+                }
+            }
+            __syncwarp();
+            const uint32_t v = area[lane];
+            if (v) {
+                len = (v >> 11) + LZ_MINM;
+                next = (v & 0x7ffu) << 5 | v >> 11;
+            }
+            // the positions that the walk visits: after k rounds, those up to 2^k - 1 tokens on
+            uint32_t to = p + len < L ? min(lane + len, 32u) : 32u;
+#pragma unroll
+            for (int k = 0; k < 5; ++k) {
+                reach |= __reduce_or_sync(GD_FULL_MASK, (reach >> lane & 1u) && to < 32u ? 1u << to : 0u);
+                const uint32_t on2 = __shfl_sync(GD_FULL_MASK, to, (int)(to & 31u));
+                if (to < 32u) to = on2;
+            }
+        } else {
+            for (uint32_t q = cur - w0; q < 32u && w0 + q < L;) {
+                const uint32_t qw = __shfl_sync(GD_FULL_MASK, w, q), qw4 = __shfl_sync(GD_FULL_MASK, w4, q);
+                const uint32_t qat = __shfl_sync(GD_FULL_MASK, at, q);
+                uint32_t best = 0;  // (length - 3) << 11 | offset
+                for (uint32_t i = __shfl_sync(GD_FULL_MASK, first, q); i < qat; i += 32) {
+                    const uint32_t c = i + lane < qat ? pos[i + lane] : w0 + q;  // itself: no match
+                    const uint32_t f = match(c, w0 + q, qw, qw4);
+                    best = max(best, __reduce_max_sync(GD_FULL_MASK, f ? (f - LZ_MINM) << 11 | (w0 + q - c) : 0u));
+                    if (best >> 11 == LZ_MAXM - LZ_MINM) break;  // later candidates are nearer
+                }
+                const uint32_t step = best ? (best >> 11) + LZ_MINM : 1u;
+                if (lane == q && best) {
+                    len = step;
+                    next = (best & 0x7ffu) << 5 | best >> 11;
+                }
+                reach |= 1u << q;
+                q += step;
+            }
+        }
+        if (!reach) break;  // the column's end
+        // ---- their bytes, and a flag byte before every 8 ----
+        const uint32_t k = __popc(reach), last = 31u - __clz(reach);
+        cur = w0 + last + __shfl_sync(GD_FULL_MASK, len, last);
+        const bool here = reach >> lane & 1u, lit = len == 1u;
+        const uint32_t long_ones = __ballot_sync(GD_FULL_MASK, here && !lit);
+        const uint32_t rank = __popc(reach & lt), g = nt + rank;
+        const uint32_t lits = __reduce_or_sync(GD_FULL_MASK, here && lit ? 1u << rank : 0u);
+        const uint64_t flags = (uint64_t)lits << nt | flag;
+        const uint32_t place = on + rank + __popc(long_ones & lt) + (g >> 3) + (nt ? 0u : 1u);
+        if (here) {
+            if ((g & 7u) == 0) out[place - 1u] = (uint8_t)(flags >> g);
+            out[place] = (uint8_t)next;
+            if (!lit) out[place + 1u] = (uint8_t)(next >> 8);
+        }
+        if (nt && lane == 0) out[flag_at] = (uint8_t)flags;
+        on += k + __popc(long_ones) + ((nt + k + 7u) >> 3) - (nt ? 1u : 0u);
+        const uint32_t open = (nt + k) & ~7u;  // the open group's first token
+        const uint32_t opener = __ballot_sync(GD_FULL_MASK, here && g == open);
+        if (opener) flag_at = __shfl_sync(GD_FULL_MASK, place, __ffs(opener) - 1) - 1u;
+        nt = (nt + k) & 7u;
+        flag = (uint32_t)(flags >> open) & 0xffu;
+        __syncwarp();
+        if (on >= LZ_OUT / 2u) {  // whole words, up to the open group
+            const uint32_t nw = (nt ? flag_at : on) >> 2;
+            over = over || 4u * (written + nw) > cap;
+            if (!over)
+                for (uint32_t i = lane; i < nw; i += 32) slot[written + i] = reinterpret_cast<const uint32_t*>(out)[i];
+            written += nw;
+            on -= 4u * nw;
+            flag_at -= 4u * nw;
+            uint8_t keep = 0;  // 3 bytes and 8 tokens at most
+            if (lane < on) keep = out[4u * nw + lane];
+            __syncwarp();
+            if (lane < on) out[lane] = keep;
+            __syncwarp();
+        }
     }
-    emit(true);
+    // the end: a reserved flag byte after a full group, zeros to a whole word
+    if (nt == 0) {
+        if (lane == 0) out[on] = 0;
+        ++on;
+    }
+    if ((on & 3u) && (on & 3u) + lane < 4u) out[on + lane] = 0;
+    __syncwarp();
+    over = over || 4u * written + ((on + 3u) & ~3u) > cap;
+    if (!over)
+        for (uint32_t i = lane; i < (on + 3u) >> 2; i += 32) slot[written + i] = reinterpret_cast<const uint32_t*>(out)[i];
     if (lane == 0) raw_len[col] = over ? 0xffffffffu : 4u * written + on;
 }
 

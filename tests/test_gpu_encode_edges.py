@@ -84,3 +84,20 @@ def test_lzss(cuda, chunk):
         for k in want.meta:
             assert np.array_equal(want.meta[k], got.meta[k]), (k, cut)
         assert np.array_equal(want.data, got.data), cut
+
+
+@pytest.mark.parametrize("chunk", [2048, 65536, 131072])
+def test_lzss_pairs(cuda, chunk):
+    """Columns of 1 to 32 distinct bytes: 32 positions with anything from a
+    few to thousands of older positions to compare, in one column a stretch of
+    each."""
+    rng = np.random.default_rng(7 * chunk)
+    n = chunk // 32
+    cols = [rng.integers(0, q + 1, n, dtype=np.uint8) for q in range(31)]
+    cols.append(np.resize(np.concatenate([rng.integers(0, k, 96, dtype=np.uint8) for k in (1, 2, 64, 4, 16, 1, 256)]), n))
+    raw = np.stack([x.reshape(-1, 4) for x in cols], 1).reshape(-1)
+    want = cc.lzss_encode(raw, chunk)
+    got = cc.encode_gpu("lzss", raw, chunk)
+    for k in want.meta:
+        assert np.array_equal(want.meta[k], got.meta[k]), k
+    assert np.array_equal(want.data, got.data)
