@@ -78,6 +78,24 @@ __global__ void __launch_bounds__(32 * G) decode_cols_kernel(const uint8_t* __re
 }  // namespace lzss
 }  // namespace gd
 
+// Whether decode_follow_kernel is the faster for n chunks of 32 L bytes.  The
+// group decoder's time is a column's serial chain, whatever runs beside it, up
+// to 15 chunks an SM; beyond that it needs fewer instructions a byte, the more
+// so the shorter the columns.  Follow against group, us:
+//   128 KiB chunks   256 MiB 1635 / 2337   512 MiB 3217 / 4172
+//    64 KiB chunks    64 MiB 331 / 586     512 MiB 2429 / 2637   1 GiB 4827 / 4793
+//    32 KiB chunks    64 MiB 328 / 351     128 MiB 631 / 649     256 MiB 1235 / 1220
+//    16 KiB chunks     8 MiB 64 / 132       16 MiB 111 / 144      32 MiB 202 / 189
+//     4 KiB chunks     1 MiB 21 / 38         2 MiB 32 / 38         4 MiB 52 / 44
+//     1 KiB chunks     1 MiB 29 / 20
+static bool follow_wins(uint32_t n, uint32_t L) {
+    int dev = 0, sms = 148;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    const uint32_t per_sm = L >= 2048u ? 60u : L >= 1024u ? 30u : L >= 512u ? 10u : L >= 128u ? 5u : 0u;
+    return n <= per_sm * (uint32_t)sms;
+}
+
 extern "C" gd_status_t gd_lzss_decode(const uint8_t* d_data, const uint64_t* d_blk_off, const uint64_t* d_col_len,
                                       const uint8_t* d_col_map, uint32_t n_chunks, uint64_t chunk_size,
                                       uint8_t* d_out, uint64_t out_n_bytes, uint32_t* d_status,
@@ -116,8 +134,10 @@ extern "C" gd_status_t gd_lzss_decode(const uint8_t* d_data, const uint64_t* d_b
     }
     // columns of up to 4 KiB, 16-byte row stores: a block per 8 columns (5 an
     // SM at 2 KiB), or per 4 where 8 columns' workspaces leave room for two
-    // blocks on an SM only (128 KiB chunks: 1.63 ms for 256 MiB)
-    if (k == 0 && chunk_size / 32 <= FMAXL && (reinterpret_cast<uintptr_t>(d_out) & 15u) == 0) {
+    // blocks on an SM only (128 KiB chunks: 1.63 ms for 256 MiB); not so many
+    // chunks that the group decoder fills the chip (follow_wins)
+    if (k == 0 && chunk_size / 32 <= FMAXL && (reinterpret_cast<uintptr_t>(d_out) & 15u) == 0 &&
+        follow_wins(n_chunks, (uint32_t)(chunk_size / 32))) {
         const uint32_t L = (uint32_t)(chunk_size / 32);
         cudaStream_t s = (cudaStream_t)stream;
         if (d_status && cudaMemsetAsync(d_status, 0, 4ull * n_chunks, s) != cudaSuccess) return GD_ERR_CUDA;
