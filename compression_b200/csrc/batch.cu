@@ -21,6 +21,7 @@
 // four warps a block and stream 3.0 ms (the largest stream alone takes 2.9).
 // Per-task %globaltimer start/end stamps (optional) are the measurements the
 // learned cost model trains on.
+#include "batch_turns.cuh"
 #include "brle_warp.cuh"
 #include "inflate_block.cuh"
 #include "lzss.cuh"
@@ -155,12 +156,7 @@ __global__ void __launch_bounds__(C::WPB * 32, C::BPS) batch_kernel(const gd_tas
                                                            int dynamic, uint32_t max_lane, uint32_t ws_bytes,
                                                            uint32_t* __restrict__ status,
                                                            uint64_t* __restrict__ timing) {
-    constexpr uint32_t WPB = C::WPB;
     extern __shared__ __align__(16) uint8_t smem[];
-    __shared__ uint32_t s_list[WPB], s_nd;  // Deflate tasks taken
-    __shared__ uint32_t s_stop, s_soon, s_end;
-    constexpr uint32_t NONE = 0xffffffffu;
-    const uint32_t lane = lane_id(), wid = threadIdx.x >> 5;
     auto done = [&](uint32_t ti, uint32_t e, uint64_t t0) {
         put_status(status, ti, e);
         if (timing) {
@@ -168,90 +164,21 @@ __global__ void __launch_bounds__(C::WPB * 32, C::BPS) batch_kernel(const gd_tas
             timing[2ull * ti + 1] = globaltimer();
         }
     };
-    // task of queue place j; NONE past the end, or for a malformed order array
-    auto look = [&](uint32_t j, bool& defl) -> uint32_t {
-        uint32_t ti = NONE;
-        if (j < n) ti = order ? order[j] : j;
-        if (ti >= n) ti = NONE;
-        defl = ti != NONE && tasks[ti].codec == GD_CODEC_DEFLATE;
-        return ti;
-    };
-    // the next task of the queue, for the calling warp; soon: a Deflate task
-    // lies in the part of the queue that the blocks will take next
-    auto pop = [&](bool& defl, bool& soon) -> uint32_t {
-        uint32_t i = 0;
-        if (lane == 0) i = atomicAdd(counter, 1u);
-        i = __shfl_sync(GD_FULL_MASK, i, 0);
-        bool d;
-        const uint32_t ti = __shfl_sync(GD_FULL_MASK, look(i + lane * (gridDim.x * WPB / 16u), d), 0);
-        const uint32_t m = __ballot_sync(GD_FULL_MASK, d);
-        defl = m & 1u;
-        soon = (m >> 1) != 0;
-        return ti;
-    };
-    if (threadIdx.x == 0) s_soon = 1;
-    for (uint32_t k = 0;; ++k) {
-        uint32_t first = NONE;  // warp 0: a task in hand
-        if (wid == 0) {
-            uint32_t nd = 0, end = !dynamic && (blockIdx.x + k * gridDim.x) * WPB >= n;
-            if (dynamic && s_soon) {
-                bool defl, soon;
-                first = pop(defl, soon);
-                __syncwarp();
-                end = first == NONE;
-                nd = defl;
-                if (lane == 0) {
-                    s_list[0] = first;
-                    s_soon = soon;
-                }
-            }
-            if (lane == 0) {
-                s_nd = nd;
-                s_end = end;
-                s_stop = 0;
-            }
-        }
-        __syncthreads();
-        if (!s_end && !s_nd) {
-            for (;;) {
-                bool defl = false, soon = false;
-                uint32_t ti = first;
-                first = NONE;
-                if (!dynamic) {
-                    ti = look((blockIdx.x + k * gridDim.x) * WPB + wid, defl);
-                } else if (ti == NONE) {
-                    if (*(volatile uint32_t*)&s_stop) break;
-                    ti = pop(defl, soon);
-                    if (ti == NONE && lane == 0) s_end = 1;
-                    if (soon && lane == 0) s_soon = 1;
-                }
-                if (ti != NONE && !defl) {
-                    const uint64_t t0 = globaltimer();
-                    const gd_task t = tasks[ti];
-                    const uint32_t e = run_task(t, max_lane, smem + wid * ws_bytes);
-                    __syncwarp();
-                    if (lane == 0) done(ti, e, t0);
-                } else if (ti != NONE && lane == 0) {
-                    s_list[atomicAdd(&s_nd, 1u)] = ti;
-                }
-                if (!dynamic || ti == NONE || defl || soon) {
-                    if (lane == 0) *(volatile uint32_t*)&s_stop = 1;
-                    break;
-                }
-            }
-        }
-        __syncthreads();
-        const uint32_t nd = s_nd, end = s_end;
-        for (uint32_t w = 0; w < nd; ++w) {
-            const uint32_t ti = s_list[w];
+    run_turns<C::WPB>(
+        n, order, counter, dynamic != 0, [&](uint32_t ti) { return tasks[ti].codec == GD_CODEC_DEFLATE; },
+        [&](uint32_t ti) {
+            const uint64_t t0 = globaltimer();
+            const gd_task t = tasks[ti];
+            const uint32_t e = run_task(t, max_lane, smem + (threadIdx.x >> 5) * ws_bytes);
+            __syncwarp();
+            if (lane_id() == 0) done(ti, e, t0);
+        },
+        [&](uint32_t ti) {
             const uint64_t t0 = globaltimer();
             const gd_task t = tasks[ti];
             const uint32_t e = deflate_task<C>(t, smem);
             if (threadIdx.x == 0) done(ti, e, t0);
-        }
-        if (end) break;
-        __syncthreads();  // the shared words are set for the next turn
-    }
+        });
 }
 
 using Kernel = void (*)(const gd_task*, uint32_t, const uint32_t*, uint32_t*, int, uint32_t, uint32_t, uint32_t*,

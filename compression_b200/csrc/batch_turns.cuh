@@ -1,0 +1,98 @@
+// batch_turns.cuh -- how the blocks of the batch decoder (batch.cu) take tasks.
+//
+// A block goes through turns: its warps decode tasks of their own, then the
+// whole block decodes the Deflate tasks that they met.  What a turn's start is
+// decided by (s_go) is written by warp 0 alone and by nothing that a turn does:
+// a word that a warp may change inside the turn, read late by another at its
+// start, lost that one's task.
+#pragma once
+#include "gd_common.cuh"
+
+namespace gd {
+namespace batch {
+
+// Runs the calling block's share of n tasks.  `order`: the queue (null: as
+// numbered).  Dynamic: tasks are taken
+// from the queue through `counter`, which starts at 0; else warp w of W takes
+// places w, w + W, ...  The callers' functions: deflate(ti): task ti is for a
+// block; warp_task(ti): decode it with the calling warp; block_task(ti): with
+// the block.
+template <uint32_t WPB, class Deflate, class WarpTask, class BlockTask>
+__device__ __forceinline__ void run_turns(uint32_t n, const uint32_t* __restrict__ order, uint32_t* counter,
+                                          bool dynamic, Deflate deflate, WarpTask warp_task, BlockTask block_task) {
+    __shared__ uint32_t s_list[WPB], s_nd;  // Deflate tasks taken
+    __shared__ uint32_t s_go, s_stop, s_soon, s_end;
+    constexpr uint32_t NONE = 0xffffffffu;
+    const uint32_t lane = lane_id(), wid = threadIdx.x >> 5, W = gridDim.x * WPB;
+    // task of queue place j: NONE past the end, or for an entry out of range
+    auto entry = [&](uint32_t j) -> uint32_t {
+        if (j >= n) return NONE;
+        const uint32_t ti = order ? order[j] : j;
+        return ti < n ? ti : NONE;
+    };
+    // the next task of the queue, for the calling warp; soon: a Deflate task
+    // lies in the part of the queue that the blocks will take next
+    auto pop = [&](bool& defl, bool& soon) -> uint32_t {
+        uint32_t i = 0;
+        if (lane == 0) i = atomicAdd(counter, 1u);
+        i = __shfl_sync(GD_FULL_MASK, i, 0);
+        const uint32_t t = entry(i + lane * (W / 16u));
+        const uint32_t m = __ballot_sync(GD_FULL_MASK, t != NONE && deflate(t));
+        defl = m & 1u;
+        soon = (m >> 1) != 0;
+        return __shfl_sync(GD_FULL_MASK, t, 0);
+    };
+    uint32_t at = blockIdx.x * WPB + wid;  // the static mapping's next place
+    if (threadIdx.x == 0) s_soon = 1;
+    for (;;) {
+        uint32_t first = NONE;  // warp 0: a task in hand
+        if (wid == 0) {
+            bool defl = false, soon = false, end = !dynamic && at >= n;
+            if (dynamic && s_soon) {
+                first = pop(defl, soon);
+                end = first == NONE;
+            }
+            if (lane == 0) {
+                s_list[0] = first;
+                s_nd = defl;
+                s_go = !defl && !end;
+                s_stop = 0;
+                s_soon = soon;
+                s_end = end;
+            }
+        }
+        __syncthreads();
+        if (s_go) {
+            for (;;) {
+                bool defl = false, soon = false;
+                uint32_t ti = first;
+                first = NONE;
+                if (!dynamic) {
+                    ti = entry(at);
+                    at += W;
+                    defl = ti != NONE && deflate(ti);
+                } else if (ti == NONE) {
+                    if (*(volatile uint32_t*)&s_stop) break;
+                    ti = pop(defl, soon);
+                }
+                if (ti != NONE && !defl) warp_task(ti);
+                const bool leave = !dynamic || ti == NONE || defl || soon;
+                if (lane == 0) {
+                    if (ti == NONE && dynamic) s_end = 1;
+                    if (soon) s_soon = 1;
+                    if (defl) s_list[atomicAdd(&s_nd, 1u)] = ti;
+                    if (leave) *(volatile uint32_t*)&s_stop = 1;
+                }
+                if (leave) break;
+            }
+        }
+        __syncthreads();
+        const uint32_t nd = s_nd, end = s_end;
+        for (uint32_t w = 0; w < nd; ++w) block_task(s_list[w]);
+        if (end) break;
+        __syncthreads();  // the shared words are set for the next turn
+    }
+}
+
+}  // namespace batch
+}  // namespace gd
