@@ -4,7 +4,9 @@
 // whole block decodes the Deflate tasks that they met.  What a turn's start is
 // decided by (s_go) is written by warp 0 alone and by nothing that a turn does:
 // a word that a warp may change inside the turn, read late by another at its
-// start, lost that one's task.
+// start, lost that one's task.  A warp branches on shared words that other
+// warps write only through one lane's reading of them, so that its lanes stay
+// together at the warp collectives.
 #pragma once
 #include "gd_common.cuh"
 
@@ -43,12 +45,11 @@ __device__ __forceinline__ void run_turns(uint32_t n, const uint32_t* __restrict
         return __shfl_sync(GD_FULL_MASK, t, 0);
     };
     uint32_t at = blockIdx.x * WPB + wid;  // the static mapping's next place
-    if (threadIdx.x == 0) s_soon = 1;
-    for (;;) {
+    for (bool begin = true;; begin = false) {
         uint32_t first = NONE;  // warp 0: a task in hand
         if (wid == 0) {
             bool defl = false, soon = false, end = !dynamic && at >= n;
-            if (dynamic && s_soon) {
+            if (dynamic && (begin || __shfl_sync(GD_FULL_MASK, s_soon, 0))) {
                 first = pop(defl, soon);
                 end = first == NONE;
             }
@@ -72,7 +73,9 @@ __device__ __forceinline__ void run_turns(uint32_t n, const uint32_t* __restrict
                     at += W;
                     defl = ti != NONE && deflate(ti);
                 } else if (ti == NONE) {
-                    if (*(volatile uint32_t*)&s_stop) break;
+                    uint32_t stop = 0;
+                    if (lane == 0) stop = *(volatile uint32_t*)&s_stop;
+                    if (__shfl_sync(GD_FULL_MASK, stop, 0)) break;
                     ti = pop(defl, soon);
                 }
                 if (ti != NONE && !defl) warp_task(ti);
@@ -84,6 +87,7 @@ __device__ __forceinline__ void run_turns(uint32_t n, const uint32_t* __restrict
                     if (leave) *(volatile uint32_t*)&s_stop = 1;
                 }
                 if (leave) break;
+                __syncwarp();
             }
         }
         __syncthreads();

@@ -12,7 +12,7 @@ import pytest
 
 ROOT = Path(__file__).resolve().parent.parent
 SIMT = ROOT / "tests" / "simt"
-LATE_WARPS = [0, 3, 4, 100, 101, 102]  # see simt::schedule
+SCHEDULES = [0, 1, 2, 3, 4, 11, 12, 100, 101]  # see simt::schedule
 
 
 def _compile(src: Path, out: Path, *flags) -> C.CDLL:
@@ -41,7 +41,7 @@ def turns(tmp_path_factory):
     return run
 
 
-@pytest.mark.parametrize("kind", LATE_WARPS)
+@pytest.mark.parametrize("kind", SCHEDULES)
 @pytest.mark.parametrize("wpb", [8, 4])
 @pytest.mark.parametrize("dynamic", [True, False])
 def test_every_task_once(turns, wpb, dynamic, kind):
