@@ -14,7 +14,7 @@ namespace gd {
 namespace batch {
 
 // Runs the calling block's share of n tasks.  `order`: the queue (null: as
-// numbered).  Dynamic: tasks are taken
+// numbered); entries out of range are passed over.  Dynamic: tasks are taken
 // from the queue through `counter`, which starts at 0; else warp w of W takes
 // places w, w + W, ...  The callers' functions: deflate(ti): task ti is for a
 // block; warp_task(ti): decode it with the calling warp; block_task(ti): with
@@ -24,25 +24,28 @@ __device__ __forceinline__ void run_turns(uint32_t n, const uint32_t* __restrict
                                           bool dynamic, Deflate deflate, WarpTask warp_task, BlockTask block_task) {
     __shared__ uint32_t s_list[WPB], s_nd;  // Deflate tasks taken
     __shared__ uint32_t s_go, s_stop, s_soon, s_end;
-    constexpr uint32_t NONE = 0xffffffffu;
+    constexpr uint32_t NONE = 0xffffffffu, BAD = 0xfffffffeu;
     const uint32_t lane = lane_id(), wid = threadIdx.x >> 5, W = gridDim.x * WPB;
-    // task of queue place j: NONE past the end, or for an entry out of range
+    // task of queue place j: NONE past the end, BAD for an entry out of range
     auto entry = [&](uint32_t j) -> uint32_t {
         if (j >= n) return NONE;
         const uint32_t ti = order ? order[j] : j;
-        return ti < n ? ti : NONE;
+        return ti < n ? ti : BAD;
     };
     // the next task of the queue, for the calling warp; soon: a Deflate task
     // lies in the part of the queue that the blocks will take next
     auto pop = [&](bool& defl, bool& soon) -> uint32_t {
-        uint32_t i = 0;
-        if (lane == 0) i = atomicAdd(counter, 1u);
-        i = __shfl_sync(GD_FULL_MASK, i, 0);
-        const uint32_t t = entry(i + lane * (W / 16u));
-        const uint32_t m = __ballot_sync(GD_FULL_MASK, t != NONE && deflate(t));
-        defl = m & 1u;
-        soon = (m >> 1) != 0;
-        return __shfl_sync(GD_FULL_MASK, t, 0);
+        for (;;) {
+            uint32_t i = 0;
+            if (lane == 0) i = atomicAdd(counter, 1u);
+            i = __shfl_sync(GD_FULL_MASK, i, 0);
+            const uint32_t t = entry(i + lane * (W / 16u));
+            const uint32_t m = __ballot_sync(GD_FULL_MASK, t < n && deflate(t));
+            const uint32_t ti = __shfl_sync(GD_FULL_MASK, t, 0);
+            defl = m & 1u;
+            soon = (m >> 1) != 0;
+            if (ti != BAD) return ti;
+        }
     };
     uint32_t at = blockIdx.x * WPB + wid;  // the static mapping's next place
     for (bool begin = true;; begin = false) {
@@ -71,6 +74,7 @@ __device__ __forceinline__ void run_turns(uint32_t n, const uint32_t* __restrict
                 if (!dynamic) {
                     ti = entry(at);
                     at += W;
+                    if (ti == BAD) ti = NONE;
                     defl = ti != NONE && deflate(ti);
                 } else if (ti == NONE) {
                     uint32_t stop = 0;

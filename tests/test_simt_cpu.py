@@ -52,3 +52,19 @@ def test_every_task_once(turns, wpb, dynamic, kind):
             for order in (None, rng.permutation(n)):
                 w, b = turns(wpb, deflate, order, dynamic, 2, kind)
                 assert (w == np.where(deflate, 0, 32)).all() and (b == np.where(deflate, 32 * wpb, 0)).all(), (n, share)
+
+
+@pytest.mark.parametrize("kind", [0, 4])
+@pytest.mark.parametrize("dynamic", [True, False])
+def test_entries_out_of_range(turns, dynamic, kind):
+    """An order entry that names no task costs nobody a task."""
+    rng = np.random.default_rng(kind)
+    n = 120
+    deflate = rng.random(n) < 0.2
+    order = rng.permutation(n).astype(np.uint32)
+    order = order[: n - 40]
+    for k in rng.choice(order.size, 20, replace=False):
+        order[k] = [n, n + 5, 0xffffffff, 0xfffffffe, 0x80000000][k % 5]
+    named = np.isin(np.arange(n), order)
+    w, b = turns(8, deflate, np.concatenate([order, np.full(40, n, np.uint32)]), dynamic, 2, kind)
+    assert (w == np.where(named & ~deflate, 32, 0)).all() and (b == np.where(named & deflate, 256, 0)).all()
