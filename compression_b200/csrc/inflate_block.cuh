@@ -301,6 +301,9 @@ struct Writer {
         if (p + tid < v0) S.win[(p + tid) & M] = s[tid];
         __syncthreads();
         flush(v0, false);
+        // a block of nearly WIN bytes or more also writes the window's place
+        // of the vector that flush reads
+        __syncthreads();
         const uint8_t* sv = s + (v0 - p);
         const uint32_t sh = (uint32_t)(reinterpret_cast<uintptr_t>(sv) & 3u) * 8u;
         const uint32_t* sw = reinterpret_cast<const uint32_t*>(sv - (sh >> 3));

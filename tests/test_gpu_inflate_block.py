@@ -2,6 +2,7 @@
 go wrong: segment, batch, placement and window edges, codes that never fall
 back into step, long runs, every block type and header, unaligned outputs.
 Bytes are exact, against zlib."""
+import struct
 import zlib
 
 import numpy as np
@@ -99,3 +100,61 @@ def test_malformed(cuda, variant):
             assert st[i] == 0 and np.array_equal(out[i * 30000:(i + 1) * 30000], raw[i * 30000:(i + 1) * 30000]), i
         elif i % 3 != 2:
             assert st[i] in (2, 3), (i, st[i])
+
+
+def _stored(n: int, size: int) -> tuple:
+    """n bytes in stored blocks of `size`, after a compressed block of 5 bytes."""
+    raw = b"abcde" + rng.bytes(n)
+    c = zlib.compressobj(6, zlib.DEFLATED, -15)
+    comp = c.compress(raw[:5]) + c.flush(zlib.Z_FULL_FLUSH)
+    for i in range(5, len(raw), size):
+        p = raw[i:i + size]
+        comp += struct.pack("<BHH", i + size >= len(raw), len(p), len(p) ^ 0xffff) + p
+    return np.frombuffer(raw, np.uint8), np.frombuffer(comp, np.uint8)
+
+
+STORED = [16384 - 33, 16384 + 7, 32768 - 16, 32768 + 40, 65535]
+
+
+@pytest.mark.parametrize("variant", [0, 1, 2, 3, 4])
+def test_stored_blocks_around_the_window(cuda, variant):
+    import compression_b200.autotune as at
+    raws, comps = zip(*[_stored(300001, size) for size in STORED for _ in range(60)])
+    off = np.concatenate([[0], np.cumsum([c.size + 3 for c in comps])])
+    data = np.zeros(int(off[-1]), np.uint8)
+    for o, c in zip(off, comps):
+        data[o:o + c.size] = c
+    oo = np.concatenate([[0], np.cumsum([r.size for r in raws])]).astype(np.uint64)
+    enc = cc.Encoded("deflate", data, int(oo[-1]), len(raws), 0,
+                     {"comp_off": off.astype(np.uint64), "comp_len": np.array([c.size for c in comps], np.uint64),
+                      "out_off": oo}, {"zlib_header": 0})
+    prev = at.set_knob(at.TUNE_INFLATE_VARIANT, variant)
+    try:
+        job = cc.DeviceJob(enc, cuda)
+        job.launch()
+        st, out = job.status(), job.output()
+    finally:
+        at.set_knob(at.TUNE_INFLATE_VARIANT, prev)
+    assert (st == 0).all() and np.array_equal(out, np.concatenate(raws))
+
+
+@pytest.mark.parametrize("long_lanes", [False, True])
+def test_stored_blocks_in_a_batch(cuda, long_lanes):
+    """By blocks of eight warps, and of four (lane streams of some 23 KB)."""
+    import torch
+    from compression_b200 import batch as B
+    items = []
+    for size in STORED * 4:
+        raw, comp = _stored(100003, size)
+        meta = {"comp_off": np.array([0, comp.size], np.uint64), "comp_len": np.array([comp.size], np.uint64),
+                "out_off": np.array([0, raw.size], np.uint64)}
+        items.append(B.Item("deflate", raw, cc.Encoded("deflate", comp, raw.size, 1, 0, meta, {"zlib_header": 0})))
+    if long_lanes:
+        v = cc.gen_rlev1_ints(7, 1 << 19)
+        items.append(B.Item("rlev1", v.view(np.uint8), cc.rlev1_encode(v, 1 << 20, 128, 4)))
+    plan = B.build_plan(items, cuda)
+    for dynamic in (True, False):
+        plan.d_out.zero_()
+        B.launch(plan, None, dynamic=dynamic)
+        torch.cuda.synchronize()
+        assert B.verify(plan)

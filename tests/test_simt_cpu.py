@@ -4,7 +4,9 @@ schedules in which chosen warps or lanes are as late as the code allows
 have had the time to change up to the next one.  A missing barrier gives a
 wrong result here, a warp that comes apart a kernel that does not end."""
 import ctypes as C
+import struct
 import subprocess
+import zlib
 from pathlib import Path
 
 import numpy as np
@@ -68,3 +70,42 @@ def test_entries_out_of_range(turns, dynamic, kind):
     named = np.isin(np.arange(n), order)
     w, b = turns(8, deflate, np.concatenate([order, np.full(40, n, np.uint32)]), dynamic, 2, kind)
     assert (w == np.where(named & ~deflate, 32, 0)).all() and (b == np.where(named & deflate, 256, 0)).all()
+
+
+@pytest.fixture(scope="module")
+def inflate(tmp_path_factory):
+    f = _compile(SIMT / "inflate_block.cpp", tmp_path_factory.mktemp("simt") / "inflate.so").inflate
+
+    def run(shape, comp: bytes, n: int, kind: int, at: int = 0):
+        """The n bytes written at an address `at` above a multiple of 16."""
+        src = np.zeros(len(comp) + 32, np.uint8)
+        s0 = -src.ctypes.data % 16
+        src[s0:s0 + len(comp)] = np.frombuffer(comp, np.uint8)
+        dst = np.full(n + 64, 0x5A, np.uint8)
+        d0 = -dst.ctypes.data % 16 + at
+        w = C.c_uint32()
+        st = f(shape, _p(src[s0:]), len(comp), _p(dst[d0:]), n, 0, kind, C.byref(w))
+        assert st == 0 and w.value == n
+        assert (dst[:d0] == 0x5A).all() and (dst[d0 + n:] == 0x5A).all()
+        return dst[d0:d0 + n]
+    return run
+
+
+def _stored(parts) -> bytes:
+    """The parts as stored blocks, after a compressed one of 5 bytes."""
+    c = zlib.compressobj(6, zlib.DEFLATED, -15)
+    out = c.compress(b"abcde") + c.flush(zlib.Z_FULL_FLUSH)
+    for i, p in enumerate(parts):
+        out += struct.pack("<BHH", i == len(parts) - 1, len(p), len(p) ^ 0xffff) + p
+    return out
+
+
+@pytest.mark.parametrize("shape,window", [(1, 65536), (2, 32768), (3, 32768), (4, 16384), (5, 16384)])
+@pytest.mark.parametrize("kind", [0, 4])
+def test_stored_blocks_around_the_window(inflate, shape, window, kind):
+    """Stored blocks of about the window's length at odd places."""
+    rng = np.random.default_rng(shape)
+    for at in (0, 3):
+        parts = [rng.bytes(min(65535, window + k)) for k in (-33, 40, 7, 100)]
+        got = inflate(shape, _stored(parts), 5 + sum(map(len, parts)), kind, at)
+        assert got.tobytes() == b"abcde" + b"".join(parts)
