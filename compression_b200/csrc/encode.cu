@@ -261,10 +261,14 @@ __global__ void __launch_bounds__(LZ_WPB * 32) lzss_column_kernel(const uint8_t*
             at = end[h] + __popc(peers & lt);
             pos[at] = (uint16_t)p;
             first = start[h];
-            if (aged)
-                while (first < at && pos[first] + LZ_HIST <= w0) ++first;  // too old for all 32, and those after
         }
         __syncwarp();
+        if (aged) {
+            // too old for all 32, and those after; the list may reach into these 32 positions
+            if (keyed)
+                while (first < at && pos[first] + LZ_HIST <= w0) ++first;
+            __syncwarp();
+        }
         if (keyed && (peers >> lane) == 1u) {  // the last of its bucket here
             end[h] = (uint16_t)(at + 1u);
             if (aged) start[h] = (uint16_t)first;

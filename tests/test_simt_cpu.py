@@ -12,6 +12,9 @@ from pathlib import Path
 import numpy as np
 import pytest
 
+from compression_b200 import codecs as cc
+from compression_b200._lib import lib
+
 ROOT = Path(__file__).resolve().parent.parent
 SIMT = ROOT / "tests" / "simt"
 SCHEDULES = [0, 1, 2, 3, 4, 11, 12, 100, 101]  # see simt::schedule
@@ -109,3 +112,31 @@ def test_stored_blocks_around_the_window(inflate, shape, window, kind):
         parts = [rng.bytes(min(65535, window + k)) for k in (-33, 40, 7, 100)]
         got = inflate(shape, _stored(parts), 5 + sum(map(len, parts)), kind, at)
         assert got.tobytes() == b"abcde" + b"".join(parts)
+
+
+@pytest.fixture(scope="module")
+def lzss_columns(tmp_path_factory):
+    text = (ROOT / "compression_b200" / "csrc" / "encode.cu").read_text()
+    tmp = tmp_path_factory.mktemp("simt")
+    (tmp / "cols.inc").write_text(text[text.index("constexpr uint32_t LZ_WPB"):text.index("// A warp per chunk: slots")])
+    return _compile(SIMT / "lzss_columns.cpp", tmp / "lzss.so", f'-DLZSS_COLUMNS="{tmp / "cols.inc"}"').lzss_columns
+
+
+@pytest.mark.parametrize("chunk", [1024, 65536, 131072])
+@pytest.mark.parametrize("kind", [0, 1, 2, 11])
+def test_lzss_columns_match_the_host_encoder(lzss_columns, chunk, kind):
+    rng = np.random.default_rng(chunk)
+    n = chunk // 32
+    text = cc.gen_markov_copy(3, n, 4096)
+    fresh = np.zeros(n, np.uint8)  # words repeated at once, not seen before
+    for p in range(0, n - 31, 32):
+        fresh[p:p + 8] = fresh[p + 10:p + 18] = rng.integers(1, 256, 8) if p % 96 == 0 else 0
+    cols = [fresh, rng.integers(0, 2, n, dtype=np.uint8), text, rng.integers(0, 12, n, dtype=np.uint8)]
+    raw = np.stack([(cols * 8)[q].reshape(-1, 4) for q in range(32)], 1).reshape(-1).copy()
+    cap = n + n // 8 + 12 & ~3
+    scratch, raw_len = np.zeros(32 * cap, np.uint8), np.zeros(32, np.uint32)
+    assert lzss_columns(_p(raw), C.c_uint64(chunk), 0, 4, _p(scratch), cap, _p(raw_len), kind) == 0
+    for q in range(4):
+        want = np.zeros(cap, np.uint8)
+        m = lib().gd_lzss_encode_stream(_p(cols[q]), n, _p(want), cap)
+        assert raw_len[q] == m and np.array_equal(scratch[q * cap:q * cap + m], want[:m]), q
