@@ -263,91 +263,102 @@ __device__ __forceinline__ uint32_t block_scan(uint32_t v, uint32_t* red, uint32
 
 // The output side of a stream.  Positions count from the 16-byte-aligned
 // address below dst, so that window words and 16-byte vectors line up with the
-// output's.  Bytes from `flushed` on are in the window only.
+// output's.  They are taken modulo 2^32 (a stream of 2^32 - 1 bytes may end
+// beyond it), so they are told apart by their differences, and the output is
+// addressed from `flushed`.  Bytes from there on are in the window only.
 template <class SmemT>
 struct Writer {
     static constexpr uint32_t NT = SmemT::NT, WIN = SmemT::WIN, M = WIN - 1, NW = NT / 32;
     static_assert((WIN & (WIN - 1)) == 0 && 2 * SmemT::TMAX + 274 <= WIN, "window");
     static_assert(SmemT::TMAX >= 258 && SmemT::TMAX % 8 == 0, "a placement holds a symbol");
     SmemT& S;
-    uint8_t* out;      // dst rounded down to 16 bytes
-    uint32_t base;     // dst - out
-    uint32_t flushed;  // position
+    uint8_t* at;       // where position `flushed` goes
+    uint32_t base;     // position of dst
+    uint32_t flushed;
 
     __device__ __forceinline__ Writer(SmemT& s, uint8_t* dst) : S(s) {
         base = (uint32_t)(reinterpret_cast<uintptr_t>(dst) & 15u);
-        out = dst - base;
+        at = dst;
         flushed = base;
+    }
+    __device__ __forceinline__ void advance(uint32_t n) {
+        at += n;
+        flushed += n;
     }
     // Write the whole vectors before `to` out; last: also the bytes after them.
     __device__ __forceinline__ void flush(uint32_t to, bool last) {
         const uint32_t tid = threadIdx.x;
         if (flushed & 15u) {  // the stream's first vector, shared with what precedes dst
-            const uint32_t e = min(to, (flushed | 15u) + 1u);
-            if (!last && (e & 15u)) return;
-            if (flushed + tid < e) out[flushed + tid] = S.win[(flushed + tid) & M];
-            flushed = e;
+            const uint32_t v = 16u - (flushed & 15u), m = min(to - flushed, v);
+            if (!last && m < v) return;
+            if (tid < m) at[tid] = S.win[(flushed + tid) & M];
+            advance(m);
         }
-        for (uint32_t v = flushed + 16u * tid; v + 16u <= to; v += 16u * NT)
-            *reinterpret_cast<uint4*>(out + v) = *reinterpret_cast<const uint4*>(S.win + (v & M));
-        flushed = max(flushed, to & ~15u);
-        if (last && flushed + tid < to) out[flushed + tid] = S.win[(flushed + tid) & M];
+        const uint32_t n = to - flushed;
+        for (uint32_t k = 16u * tid; k + 16u <= n; k += 16u * NT)
+            *reinterpret_cast<uint4*>(at + k) = *reinterpret_cast<const uint4*>(S.win + ((flushed + k) & M));
+        advance(n & ~15u);
+        if (last && tid < (n & 15u)) at[tid] = S.win[(flushed + tid) & M];
     }
     // m stored bytes from s to position p.  Whole vectors go straight to the
     // output and the window, four in flight a thread.
     __device__ __forceinline__ void stored(const uint8_t* __restrict__ s, uint32_t m, uint32_t p) {
         const uint32_t tid = threadIdx.x;
-        const uint32_t e = p + m, v0 = min(e, (p + 15u) & ~15u), v1 = max(v0, e & ~15u);
-        if (p + tid < v0) S.win[(p + tid) & M] = s[tid];
+        // whole vectors of the output: [v0, v1) of the m bytes
+        const uint32_t v0 = min(m, (0u - p) & 15u), r = (p + m) & 15u, v1 = m >= v0 + r ? m - r : v0;
+        if (tid < v0) S.win[(p + tid) & M] = s[tid];
         __syncthreads();
-        flush(v0, false);
+        flush(p + v0, false);
         // a block of nearly WIN bytes or more also writes the window's place
         // of the vector that flush reads
         __syncthreads();
-        const uint8_t* sv = s + (v0 - p);
+        const uint8_t* sv = s + v0;
         const uint32_t sh = (uint32_t)(reinterpret_cast<uintptr_t>(sv) & 3u) * 8u;
         const uint32_t* sw = reinterpret_cast<const uint32_t*>(sv - (sh >> 3));
+        const uint32_t n = v1 - v0;
 #pragma unroll 4
-        for (uint32_t v = v0 + 16u * tid; v + 16u <= v1; v += 16u * NT) {
-            const uint32_t* q = sw + ((v - v0) >> 2);
+        for (uint32_t k = 16u * tid; k < n; k += 16u * NT) {
+            const uint32_t* q = sw + (k >> 2);
             uint32_t w[5];
 #pragma unroll
             for (int i = 0; i < 4; ++i) w[i] = __ldg(q + i);
             w[4] = sh ? __ldg(q + 4) : 0u;
             const uint4 x = make_uint4(__funnelshift_r(w[0], w[1], sh), __funnelshift_r(w[1], w[2], sh),
                                        __funnelshift_r(w[2], w[3], sh), __funnelshift_r(w[3], w[4], sh));
-            *reinterpret_cast<uint4*>(out + v) = x;
-            if (v + WIN >= v1) *reinterpret_cast<uint4*>(S.win + (v & M)) = x;  // the newest WIN bytes
+            *reinterpret_cast<uint4*>(at + k) = x;
+            if (k + WIN >= n) *reinterpret_cast<uint4*>(S.win + ((p + v0 + k) & M)) = x;  // the newest WIN bytes
         }
-        if (v1 > v0) flushed = v1;
+        advance(n);
         __syncthreads();  // the tail's window bytes may replace ones the loop stored
-        if (v1 + tid < e) S.win[(v1 + tid) & M] = s[v1 - p + tid];
+        if (v1 + tid < m) S.win[(p + v1 + tid) & M] = s[v1 + tid];
         __syncthreads();
     }
-    // Bytes [o, e) from d bytes before them (e - o <= d) with W lanes, the
-    // caller being lane `sub`.  at(x): the aligned source word at position x.
-    template <class At>
-    __device__ __forceinline__ void copy_words(uint32_t o, uint32_t e, uint32_t d, uint32_t sub, uint32_t W, At at) {
+    // Bytes [o, e) after position q0 (a multiple of 4) from d bytes before them
+    // (e - o <= d) with W lanes, the caller being lane `sub`.  word(x): the
+    // aligned source word at position x.
+    template <class Word>
+    __device__ __forceinline__ void copy_words(uint32_t q0, uint32_t o, uint32_t e, uint32_t d, uint32_t sub, uint32_t W,
+                                               Word word) {
         const uint32_t o4 = (o + 3u) & ~3u, e4 = e & ~3u;
         // up to 3 bytes before the first whole word and after the last: lanes 0-3 and 4-7
         const uint32_t x = sub < 4u ? o + sub : max(e4, o4) + sub - 4u;
         const bool edge = sub < 4u ? x < min(o4, e) : sub < 8u && x < e;
         uint32_t v = 0;
-        if (edge) v = at((x - d) & ~3u) >> (8u * ((x - d) & 3u));
+        if (edge) v = word((q0 + x - d) & ~3u) >> (8u * ((x - d) & 3u));
         const uint32_t sh = ((0u - d) & 3u) * 8u;
         for (uint32_t q = o4 + 4u * sub; q < e4; q += 8u * W) {
-            const uint32_t s0 = (q - d) & ~3u, s1 = s0 + 4u * W;
+            const uint32_t s0 = (q0 + q - d) & ~3u, s1 = s0 + 4u * W;
             const bool two = q + 4u * W < e4;
-            const uint32_t a0 = at(s0), b0 = at(s0 + 4u);
+            const uint32_t a0 = word(s0), b0 = word(s0 + 4u);
             uint32_t a1 = 0, b1 = 0;
             if (two) {
-                a1 = at(s1);
-                b1 = at(s1 + 4u);
+                a1 = word(s1);
+                b1 = word(s1 + 4u);
             }
-            *reinterpret_cast<uint32_t*>(S.win + (q & M)) = __funnelshift_r(a0, b0, sh);
-            if (two) *reinterpret_cast<uint32_t*>(S.win + ((q + 4u * W) & M)) = __funnelshift_r(a1, b1, sh);
+            *reinterpret_cast<uint32_t*>(S.win + ((q0 + q) & M)) = __funnelshift_r(a0, b0, sh);
+            if (two) *reinterpret_cast<uint32_t*>(S.win + ((q0 + q + 4u * W) & M)) = __funnelshift_r(a1, b1, sh);
         }
-        if (edge) S.win[x & M] = (uint8_t)v;
+        if (edge) S.win[(q0 + x) & M] = (uint8_t)v;
     }
     // from[k] = k - d for k in [lo, hi), by W lanes or threads
     __device__ __forceinline__ void fill(uint32_t lo, uint32_t hi, uint32_t d, uint32_t sub, uint32_t W) {
@@ -368,13 +379,14 @@ struct Writer {
         if (o < in0) {
             const uint32_t x = min(e, in0);
             if (d + T <= WIN + o - z) {
-                copy_words(q0 + o, q0 + x, d, sub, W,
+                copy_words(q0, o, x, d, sub, W,
                            [&](uint32_t q) { return *reinterpret_cast<const uint32_t*>(S.win + (q & M)); });
             } else {
                 // the placement's later bytes may have taken the source's
                 // place in the window: read the output
-                copy_words(q0 + o, q0 + x, d, sub, W,
-                           [&](uint32_t q) { return *reinterpret_cast<const uint32_t*>(out + q); });
+                copy_words(q0, o, x, d, sub, W, [&](uint32_t q) {
+                    return *reinterpret_cast<const uint32_t*>(at + (int32_t)(q - flushed));
+                });
             }
         }
         if (in0 < e) {
@@ -441,7 +453,7 @@ struct Writer {
                         S.take_c = start ? c : c + 1u;
                     }
                 } else if (len) {
-                    if (!lit && (x >> 9) >= opos + o)
+                    if (!lit && (x >> 9) >= o && (x >> 9) - o >= opos)
                         atomicMin(&S.bad, 16u * j + ST_CORRUPT);
                     else if (o + len > room)
                         atomicMin(&S.bad, 16u * j + ST_OVERRUN);
@@ -522,11 +534,10 @@ static __device__ __forceinline__ uint32_t stream_block(const uint8_t* __restric
     // the 16-byte-aligned view of the stream: it starts at view byte sh
     const uint32_t sh = (uint32_t)(reinterpret_cast<uintptr_t>(src) & 15u);
     const uint8_t* src_al = src - sh;
-    const uint32_t span = clen + sh;  // bytes of the view we may use
-    const uint64_t bend = (uint64_t)span * 8u;
+    const uint64_t span = (uint64_t)clen + sh;  // bytes of the view we may use
+    const uint64_t bend = span * 8u;
     uint64_t bp = (uint64_t)sh * 8u;  // next bit of the view
     uint32_t opos = 0;                // output bytes so far
-    olen = min(olen, 0xffffffe0u);    // output positions (Writer) stay below 2^32
 
     if (zlib_hdr == 1) {
         // zlib (RFC 1950): CMF, FLG; no preset dictionary
@@ -563,8 +574,8 @@ static __device__ __forceinline__ uint32_t stream_block(const uint8_t* __restric
     // bit 0 of S.in is bit b0 of the view
     uint64_t b0 = 0;
     auto stage = [&]() {
-        const uint32_t from = (uint32_t)(bp >> 3) & ~15u;
-        const uint32_t n = min(span - from, SmemT::IN_BYTES);
+        const uint64_t from = (bp >> 3) & ~15ull;
+        const uint32_t n = (uint32_t)min((unsigned long long)(span - from), (unsigned long long)SmemT::IN_BYTES);
         __syncthreads();  // the last readers of S.in
         for (uint32_t i = 16u * tid; i < n; i += 16u * NT) {
             // whole 16-byte words; the ragged end byte by byte
@@ -575,7 +586,7 @@ static __device__ __forceinline__ uint32_t stream_block(const uint8_t* __restric
                 for (uint32_t k = i; k < n; ++k) reinterpret_cast<uint8_t*>(S.in)[k] = src_al[from + k];
             }
         }
-        b0 = (uint64_t)from * 8u;
+        b0 = from * 8u;
         __syncthreads();
     };
     // n <= 25 bits at bp (the same on every thread); false at the end of the input
@@ -613,7 +624,7 @@ static __device__ __forceinline__ uint32_t stream_block(const uint8_t* __restric
                 err = ST_CORRUPT;
                 break;
             }
-            if (ln) wr.stored(src + ((uint32_t)(bp >> 3) - sh), ln, opos + wr.base);
+            if (ln) wr.stored(src + ((bp >> 3) - sh), ln, opos + wr.base);
             bp += 8ull * ln;
             opos += ln;
             continue;

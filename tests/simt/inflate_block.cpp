@@ -33,3 +33,22 @@ extern "C" int inflate(int shape, const uint8_t* src, uint32_t clen, uint8_t* ds
         default: return go<Smem<4, 16384, 2048, 8032>>(src, clen, dst, olen, hdr, kind, written);
     }
 }
+
+// A Writer at position `start` puts n bytes, byte i of them src[i], to dst:
+// through the window, or as stored bytes.
+extern "C" int write_at(uint32_t start, const uint8_t* src, uint32_t n, uint8_t* dst, int stored, uint32_t kind) {
+    using S = Smem<8, 16384, 2048, 8032>;
+    static S smem;
+    const bool ok = simt::run(S::NT, 0, 1, simt::schedule(S::NT, kind), [&] {
+        Writer<S> w(smem, dst);
+        w.flushed = start;
+        if (stored) {
+            w.stored(src, n, start);
+        } else {
+            for (uint32_t i = threadIdx.x; i < n; i += S::NT) smem.win[(start + i) % S::WIN] = src[i];
+            __syncthreads();
+        }
+        w.flush(start + n, true);
+    });
+    return ok ? 0 : 1;
+}

@@ -158,3 +158,24 @@ def test_stored_blocks_in_a_batch(cuda, long_lanes):
         B.launch(plan, None, dynamic=dynamic)
         torch.cuda.synchronize()
         assert B.verify(plan)
+
+
+def test_largest_stream(cuda):
+    """A stream of 2^32 - 1 bytes, the most an entry point takes."""
+    n, mid = 2**32 - 1, 16 << 20
+    head, tail = rng.bytes(70000), rng.bytes(70001)
+    c = zlib.compressobj(6, zlib.DEFLATED, -15)
+    first = c.compress(head) + c.flush(zlib.Z_FULL_FLUSH)
+    zeros = c.compress(bytes(mid)) + c.flush(zlib.Z_FULL_FLUSH)
+    k, rest = divmod(n - len(head) - len(tail), mid)
+    comp = np.frombuffer(first + zeros * k + c.compress(bytes(rest) + tail) + c.flush(), np.uint8)
+    enc = cc.Encoded("deflate", comp, n, 1, 0,
+                     {"comp_off": np.array([0, comp.size], np.uint64), "comp_len": np.array([comp.size], np.uint64),
+                      "out_off": np.array([0, n], np.uint64)}, {"zlib_header": 0})
+    job = cc.DeviceJob(enc, cuda)
+    job.launch()
+    assert (job.status() == 0).all()
+    out = job.d_out[:n]
+    assert out[:len(head)].cpu().numpy().tobytes() == head and out[n - len(tail):].cpu().numpy().tobytes() == tail
+    for a in range(len(head), n - len(tail), 1 << 30):
+        assert not out[a:min(a + (1 << 30), n - len(tail))].any()

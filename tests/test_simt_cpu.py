@@ -77,7 +77,7 @@ def test_entries_out_of_range(turns, dynamic, kind):
 
 @pytest.fixture(scope="module")
 def inflate(tmp_path_factory):
-    f = _compile(SIMT / "inflate_block.cpp", tmp_path_factory.mktemp("simt") / "inflate.so").inflate
+    lib_ = _compile(SIMT / "inflate_block.cpp", tmp_path_factory.mktemp("simt") / "inflate.so")
 
     def run(shape, comp: bytes, n: int, kind: int, at: int = 0):
         """The n bytes written at an address `at` above a multiple of 16."""
@@ -87,10 +87,11 @@ def inflate(tmp_path_factory):
         dst = np.full(n + 64, 0x5A, np.uint8)
         d0 = -dst.ctypes.data % 16 + at
         w = C.c_uint32()
-        st = f(shape, _p(src[s0:]), len(comp), _p(dst[d0:]), n, 0, kind, C.byref(w))
+        st = lib_.inflate(shape, _p(src[s0:]), len(comp), _p(dst[d0:]), n, 0, kind, C.byref(w))
         assert st == 0 and w.value == n
         assert (dst[:d0] == 0x5A).all() and (dst[d0 + n:] == 0x5A).all()
         return dst[d0:d0 + n]
+    run.write_at = lib_.write_at
     return run
 
 
@@ -140,3 +141,17 @@ def test_lzss_columns_match_the_host_encoder(lzss_columns, chunk, kind):
         want = np.zeros(cap, np.uint8)
         m = lib().gd_lzss_encode_stream(_p(cols[q]), n, _p(want), cap)
         assert raw_len[q] == m and np.array_equal(scratch[q * cap:q * cap + m], want[:m]), q
+
+
+@pytest.mark.parametrize("stored", [0, 1])
+def test_output_positions_past_32_bits(inflate, stored):
+    """The last bytes of a stream of up to 2^32 - 1 bytes, whose output may
+    start up to 15 bytes after a multiple of 16."""
+    rng = np.random.default_rng(stored)
+    for start in (2**32 - 8192, 2**32 - 4096 - 5, 2**32 - 16, 2**32 - 1, 5):
+        for n in (1, 15, 16, 33, 4095, 8190):
+            src, dst = rng.integers(0, 256, n + 32, dtype=np.uint8), np.full(n + 64, 0x5A, np.uint8)
+            s0, d0 = -src.ctypes.data % 16, -dst.ctypes.data % 16 + start % 16
+            assert inflate.write_at(start % 2**32, _p(src[s0:]), n, _p(dst[d0:]), stored, 4) == 0
+            assert np.array_equal(dst[d0:d0 + n], src[s0:s0 + n])
+            assert (dst[:d0] == 0x5A).all() and (dst[d0 + n:] == 0x5A).all(), (start, n)
