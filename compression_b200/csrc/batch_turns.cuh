@@ -51,7 +51,7 @@ __device__ __forceinline__ void run_turns(uint32_t n, const uint32_t* __restrict
     for (bool begin = true;; begin = false) {
         uint32_t first = NONE;  // warp 0: a task in hand
         if (wid == 0) {
-            bool defl = false, soon = false, end = !dynamic && at >= n;
+            bool defl = false, soon = false, end = false;
             if (dynamic && (begin || __shfl_sync(GD_FULL_MASK, s_soon, 0))) {
                 first = pop(defl, soon);
                 end = first == NONE;
@@ -72,9 +72,11 @@ __device__ __forceinline__ void run_turns(uint32_t n, const uint32_t* __restrict
                 uint32_t ti = first;
                 first = NONE;
                 if (!dynamic) {
-                    ti = entry(at);
-                    at += W;
-                    if (ti == BAD) ti = NONE;
+                    // a warp goes on to its next Deflate task, or its end
+                    do {
+                        ti = entry(at);
+                        at += W;
+                    } while (ti == BAD);
                     defl = ti != NONE && deflate(ti);
                 } else if (ti == NONE) {
                     uint32_t stop = 0;
@@ -83,7 +85,7 @@ __device__ __forceinline__ void run_turns(uint32_t n, const uint32_t* __restrict
                     ti = pop(defl, soon);
                 }
                 if (ti != NONE && !defl) warp_task(ti);
-                const bool leave = !dynamic || ti == NONE || defl || soon;
+                const bool leave = ti == NONE || defl || soon;
                 if (lane == 0) {
                     if (ti == NONE && dynamic) s_end = 1;
                     if (soon) s_soon = 1;
@@ -95,7 +97,7 @@ __device__ __forceinline__ void run_turns(uint32_t n, const uint32_t* __restrict
             }
         }
         __syncthreads();
-        const uint32_t nd = s_nd, end = s_end;
+        const uint32_t nd = s_nd, end = dynamic ? s_end : nd == 0;
         for (uint32_t w = 0; w < nd; ++w) block_task(s_list[w]);
         if (end) break;
         __syncthreads();  // the shared words are set for the next turn
