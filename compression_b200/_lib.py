@@ -47,6 +47,7 @@ SIGNATURES = {
     "gd_mlp_train_step": (i32, [vp, vp, vp, vp, vp, vp, u32, C.c_float, C.c_float, C.c_float, C.c_float, u32, vp,
                                 vp, vp]),
     "gd_free": (None, [vp]),
+    "gd_buffer_bytes": (u64, [vp]),
     "gd_brle_decompress": (i32, [vp, u64, C.POINTER(vp), u64p]),
     "gd_rlev1_decompress": (i32, [vp, u64, vp, u64, vp, u64, u32, u32, u64, C.POINTER(vp), u64p]),
     "gd_rlev2_decompress": (i32, [vp, u64, u64, vp, vp, u32, u64, C.POINTER(vp), u64p]),

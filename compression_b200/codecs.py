@@ -513,29 +513,34 @@ class _Lent:
     result array uses in place; gd_free takes it back when the array and its
     views are gone.  Copying a result out of page-locked memory took as long
     as the rest of a 3 MB call (0.18 of 0.36 ms).  Bounded, because page-locked
-    memory is scarce: results beyond the limits are copied."""
+    memory is scarce: results beyond the limits are copied.  What counts is the
+    buffer, which may be longer than the result: the cache hands out the
+    smallest one that is large enough."""
     MAX_BUFFERS, MAX_BYTES = 4, 256 << 20
     _lock = threading.RLock()  # __del__ may run inside take()
     _buffers = _bytes = 0
 
     @classmethod
-    def take(cls, ptr: int, n: int):
-        """The array over n bytes at ptr, or None if too much is lent already."""
+    def take(cls, ptr: int, n: int, capacity: int = 0):
+        """The array over n bytes at ptr, a buffer of `capacity` bytes (0: of
+        n), or None if too much is lent already."""
+        size = max(n, capacity)
         with cls._lock:
-            if cls._buffers >= cls.MAX_BUFFERS or cls._bytes + n > cls.MAX_BYTES:
+            if cls._buffers >= cls.MAX_BUFFERS or cls._bytes + size > cls.MAX_BYTES:
                 return None
             cls._buffers += 1
-            cls._bytes += n
+            cls._bytes += size
         o = cls()
-        o.ptr, o.n, o.free = ptr, n, lib().gd_free
+        o.ptr, o.size, o.free = C.c_void_p(ptr), size, lib().gd_free
         o.__array_interface__ = {"data": (ptr, False), "shape": (n,), "typestr": "|u1", "version": 3}
         return np.asarray(o)
 
     def __del__(self):
-        with _Lent._lock:
-            _Lent._buffers -= 1
-            _Lent._bytes -= self.n
-        self.free(C.c_void_p(self.ptr))
+        cls = type(self)  # at interpreter exit the module's names may be gone
+        with cls._lock:
+            cls._buffers -= 1
+            cls._bytes -= self.size
+        self.free(self.ptr)
 
 
 _PINNED_KEEP: list = []  # pinned tensors backing the numpy views below
@@ -622,7 +627,7 @@ def decode_host(enc: Encoded, keep: bool = True) -> np.ndarray:
     check(rc, f"{enc.codec} host decompress")
     res = None
     if keep and n.value:
-        res = _Lent.take(out.value, n.value)
+        res = _Lent.take(out.value, n.value, L.gd_buffer_bytes(out))
         if res is not None:
             return res
     if keep:

@@ -87,6 +87,11 @@ struct PinnedCache {
         live[p] = cap;
         return p;
     }
+    size_t bytes(const void* p) {  // 0: not handed out from here
+        std::lock_guard<std::mutex> g(m);
+        auto it = live.find(const_cast<void*>(p));
+        return it == live.end() ? 0 : it->second;
+    }
     bool put(void* p) {
         std::lock_guard<std::mutex> g(m);
         auto it = live.find(p);
@@ -236,6 +241,8 @@ const char* gd_status_string(int s) {
 void gd_free(void* p) {
     if (p && !pinned().put(p)) free(p);
 }
+
+uint64_t gd_buffer_bytes(const void* p) { return p ? pinned().bytes(p) : 0; }
 
 // ---------------------------------------------------------------------------
 gd_status_t gd_brle_decompress(const uint8_t* in, uint64_t in_n_bytes, uint8_t** out, uint64_t* out_n_bytes) {

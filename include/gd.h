@@ -340,6 +340,9 @@ gd_status_t gd_mlp_train_step(float* d_params, float* d_m, float* d_v, const flo
 
 /* Release a buffer returned by a gd_*_decompress call. */
 void gd_free(void* p);
+/* Bytes of the page-locked buffer p that a host call returned: at least its
+ * result's (buffers are recycled).  0 if p is none. */
+uint64_t gd_buffer_bytes(const void* p);
 
 /* brle::decompress_gpu (include/brle/brle.h:305-342).
  * in: [u32 n_ptr][u64 ptr[n_ptr]][u64 total][data], chunk size 256 KiB. */
