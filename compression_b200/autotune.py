@@ -52,6 +52,11 @@ KNOBS = {
     "lzss": (TUNE_LZSS_WARPS_PER_BLOCK, [0, 4, 512, 256]),
 }
 
+# codec -> revision of its knob's values; remembered choices of another one (1
+# where none is noted) name other kernels.  deflate 2: 1 - 4 are the block
+# decoder's shapes; in 1 they, and 5 - 14, were warp and warp-pair shapes.
+REVISION = {"deflate": 2}
+
 
 def set_knob(key: int, value: int) -> int:
     prev = lib().gd_tune_set(key, value)
@@ -104,9 +109,10 @@ class Tuner:
         return f"{self.name}|{codec}|{size_bucket(nbytes)}"
 
     def apply(self, codec: str, nbytes: int) -> bool:
-        """Set the remembered knob for this codec and size; False if none."""
+        """Set the remembered knob for this codec and size; False if none, or
+        if its values meant other kernels when it was remembered."""
         r = self.results.get(self.key(codec, nbytes))
-        if r is None or codec not in KNOBS:
+        if r is None or codec not in KNOBS or r.get("revision", 1) != REVISION.get(codec, 1):
             return False
         set_knob(KNOBS[codec][0], int(r["value"]))
         return True
@@ -138,7 +144,8 @@ class Tuner:
             times[v] = _time_ms(job.launch, reps, flush)
         best = min(times, key=times.get)
         set_knob(knob, best)
-        res = {"codec": codec, "knob": knob, "value": int(best), "ms": {str(k): round(t, 4) for k, t in times.items()}}
+        res = {"codec": codec, "knob": knob, "value": int(best), "revision": REVISION.get(codec, 1),
+               "ms": {str(k): round(t, 4) for k, t in times.items()}}
         self.results[self.key(codec, job.enc.n_out)] = res
         return res
 
