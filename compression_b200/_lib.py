@@ -39,6 +39,7 @@ SIGNATURES = {
     "gd_copy_uncompressed_blocks": (i32, [vp, i32, vp]),
     "gd_batch_decode": (i32, [vp, u32, vp, i32, u32, u32, vp, vp, vp, vp]),
     "gd_batch_warps": (u32, [u32, u32]),
+    "gd_batch_block_warps": (u32, [u32]),
     "gd_batch_decode_lpt_noalloc": (i32, [vp, u32, vp, u32, u32, vp, vp]),
     "gd_tune_set": (i32, [i32, i32]),
     "gd_tune_get": (i32, [i32]),

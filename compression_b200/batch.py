@@ -218,6 +218,12 @@ def n_warps(plan: Plan, blocks_per_sm: int = 0) -> int:
     return int(lib().gd_batch_warps(plan.max_lane, blocks_per_sm))
 
 
+def task_warps(plan: Plan) -> np.ndarray:
+    """Warps that work on each task: a block's on a Deflate task, else one."""
+    block = int(lib().gd_batch_block_warps(plan.max_lane))
+    return np.where(plan.tasks["codec"] == CODEC_ID["deflate"], block, 1)
+
+
 def verify(plan: Plan, expect: dict | None = None) -> bool:
     """Every task OK and every item's output equal to its raw column, or to
     expect[item index] where given (the reference decoder's output for items

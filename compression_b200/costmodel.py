@@ -2,10 +2,11 @@
 
 The model is the FP32 MLP 16 -> 64 -> 64 -> 1 of csrc/mlp.cu, trained on the
 GPU by the library's own kernels (gd_mlp_train_step: forward, backward and
-Adam in one launch per mini-batch) to predict log(decode time in ns) of a
-batch task from its 16 header features (compression_b200.batch.task_features).
-The training data are per-task times the batch decoder measures itself
-(%globaltimer stamps around every task).
+Adam in one launch per mini-batch) to predict the log of a batch task's cost
+(its decode time in ns times the warps that work on it) from its 16 header
+features (compression_b200.batch.task_features).  The training data are
+per-task times the batch decoder measures itself (%globaltimer stamps around
+every task).
 
 Scheduling: tasks are sorted by predicted cost, longest first, and fed to the
 persistent decoder's work queue -- LPT list scheduling.  The lane tasks of one
@@ -15,7 +16,7 @@ the queue and run side by side: each of them reads 4 bytes of every 128-byte
 row of the block, and when they run apart every one of them fetches the rows
 again (ordering every task by its own measured time was slower than ordering
 by output bytes for that reason).  Inside bands of a factor of 2 of
-predicted time the order runs one codec after another, so that an SM's warps
+predicted cost the order runs one codec after another, so that an SM's warps
 mostly run one decoder's code: the batch kernel holds all five decoders,
 more code than the instruction cache keeps.  The static mapping (task i ->
 warp i mod W) remains the fallback.
@@ -77,11 +78,11 @@ class CostModel:
                                       C.c_void_p(d_out.data_ptr()), C.c_void_p(s)), "gd_mlp_predict")
 
     def predict(self, X: np.ndarray) -> np.ndarray:
-        """Predicted log(ns) per row of raw features X."""
+        """Predicted log(cost in warp-ns) per row of raw features X."""
         return self.predict32(X).astype(np.float64)
 
     def predict32(self, X: np.ndarray) -> np.ndarray:
-        """Predicted log(ns) in float32, computed as the scheduling graph does
+        """Predicted log(cost) in float32, computed as the scheduling graph does
         (network output + mean target, in float32)."""
         torch = self.torch
         d_x = torch.from_numpy(self._norm(X)).to(self.dev)
@@ -103,7 +104,7 @@ class CostModel:
 
     def train(self, X: np.ndarray, y: np.ndarray, epochs: int = 20, batch: int = 256, lr: float = 2e-3,
               seed: int = 0, weights: np.ndarray | None = None) -> list[float]:
-        """Adam on log-time targets; returns the mean loss of every epoch.
+        """Adam on log-cost targets; returns the mean loss of every epoch.
         weights (optional, one per row): every epoch draws its n rows with
         replacement in proportion to them (so the squared error of a row
         counts in proportion to its weight); without them each row is seen
@@ -217,8 +218,12 @@ def lpt_order(cost: np.ndarray, groups: np.ndarray | None = None, codec: np.ndar
 
 
 def measure_tasks(plan: B.Plan, seed: int = 0, reps: int = 1) -> np.ndarray:
-    """Per-task decode times (ns) measured by the batch decoder itself, in a
-    random task order through the work queue (median over reps)."""
+    """What each task costs, in warp-nanoseconds: its decode time, measured by
+    the batch decoder itself in a random task order through the work queue
+    (median over reps), times the warps that it keeps busy.  (A Deflate task
+    holds all warps of a block.  Ordered by its time alone it starts late, when
+    the other blocks are on short tasks: 4 GiB of mixed items in the order of
+    their measured times 20.1 ms, in that of their costs 17.8.)"""
     import torch
     n = plan.tasks.size
     rng = np.random.default_rng(seed)
@@ -228,7 +233,7 @@ def measure_tasks(plan: B.Plan, seed: int = 0, reps: int = 1) -> np.ndarray:
         B.launch(plan, order, dynamic=True, timing=True)
         torch.cuda.synchronize()
         ds.append(B.task_durations_ns(plan))
-    return np.median(np.stack(ds), axis=0)
+    return np.median(np.stack(ds), axis=0) * B.task_warps(plan)
 
 
 class GraphSchedule:

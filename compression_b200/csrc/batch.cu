@@ -226,6 +226,10 @@ extern "C" gd_status_t gd_batch_decode(const gd_task* d_tasks, uint32_t n_tasks,
     return cudaGetLastError() == cudaSuccess ? GD_OK : GD_ERR_CUDA;
 }
 
+extern "C" uint32_t gd_batch_block_warps(uint32_t max_lane_bytes) {
+    return gd::batch::shape(max_lane_bytes, 0).threads / 32u;
+}
+
 extern "C" uint32_t gd_batch_warps(uint32_t max_lane_bytes, uint32_t blocks_per_sm) {
     using namespace gd::batch;
     const Launch l = shape(max_lane_bytes, blocks_per_sm);

@@ -255,6 +255,8 @@ gd_status_t gd_task_features(const gd_task* d_tasks, uint32_t n_tasks, float* d_
 
 /* Number of warps gd_batch_decode runs with for these parameters. */
 uint32_t gd_batch_warps(uint32_t max_lane_bytes, uint32_t blocks_per_sm);
+/* Warps of one of its blocks, which decode a Deflate task together. */
+uint32_t gd_batch_block_warps(uint32_t max_lane_bytes);
 
 /*
  * No counterpart in the reference.  gd_batch_decode with longest-first

@@ -229,3 +229,13 @@ def test_header_features_match_host_walk(cuda):
         want = [np.log2(1 + units), share, dens, 0.0]
         assert np.allclose(H[ti], want, rtol=1e-5, atol=1e-5), (it.codec, ti, H[ti], want)
     assert set(np.unique(T["codec"])) == {0, 1, 2, 3, 4}
+
+
+def test_measured_costs_count_a_blocks_warps(batch):
+    """A Deflate task keeps every warp of a block busy."""
+    cost = measure_tasks(batch, seed=3)
+    ns = B.task_durations_ns(batch)
+    deflate = batch.tasks["codec"] == B.CODEC_ID["deflate"]
+    assert 0 < deflate.sum() < deflate.size
+    assert np.array_equal(cost[~deflate], ns[~deflate])
+    assert np.array_equal(cost[deflate], 8 * ns[deflate])  # lanes this short: blocks of 8 warps
