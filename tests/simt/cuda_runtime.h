@@ -71,7 +71,7 @@ struct Block {
     ucontext_t end;
     jmp_buf main;
     uint32_t cur = 0, live = 0, at = 0;   // the fiber that runs; those not done; those at the block barrier
-    uint32_t or_in = 0, or_out = 0;
+    uint32_t or_in = 0, or_out = 0, sum_in = 0, sum_out = 0;
     bool diverged = false;
     std::vector<uint32_t> by, rank;       // fibers by priority, and a fiber's place there
     std::vector<uint64_t> ready;          // bit of a place: its fiber can run
@@ -83,6 +83,7 @@ struct Block {
     }
 };
 inline Block* B = nullptr;
+inline uint64_t barriers = 0;  // block barriers opened so far
 
 inline void leave() {
     if (!_setjmp(B->f[B->cur].at)) _longjmp(B->main, 1);
@@ -92,7 +93,9 @@ inline void leave() {
 inline void check_block() {
     if (!B->live || B->at < B->live) return;
     B->or_out = B->or_in;
-    B->or_in = B->at = 0;
+    ++barriers;
+    B->sum_out = B->sum_in;
+    B->or_in = B->sum_in = B->at = 0;
     for (uint32_t t = 0; t < B->f.size(); ++t)
         if (B->f[t].state == AT_BLOCK) B->set(t, RUN);
 }
@@ -202,6 +205,7 @@ inline T warp_op(int op, T v, const std::function<uint64_t(const uint64_t*, uint
 }
 inline uint32_t block_op(uint32_t v) {
     B->or_in |= v;
+    B->sum_in += v;
     B->set(B->cur, AT_BLOCK);
     ++B->at;
     check_block();
@@ -220,6 +224,10 @@ inline uint32_t fold(int op, uint32_t v, F g) {
 
 inline void __syncthreads() { simt::block_op(0); }
 inline int __syncthreads_or(int p) { return simt::block_op(p != 0) != 0; }
+inline int __syncthreads_count(int p) {
+    simt::block_op(p != 0);
+    return simt::B->sum_out;
+}
 inline void __syncwarp() {
     simt::warp_op<uint32_t>(1, 0, [](const uint64_t*, uint32_t) { return 0; });
 }

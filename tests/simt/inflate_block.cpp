@@ -34,6 +34,8 @@ extern "C" int inflate(int shape, const uint8_t* src, uint32_t clen, uint8_t* ds
     }
 }
 
+extern "C" uint64_t barriers() { return simt::barriers; }
+
 // A Writer at position `start` puts n bytes, byte i of them src[i], to dst:
 // through the window, or as stored bytes.
 extern "C" int write_at(uint32_t start, const uint8_t* src, uint32_t n, uint8_t* dst, int stored, uint32_t kind) {

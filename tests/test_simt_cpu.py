@@ -92,6 +92,8 @@ def inflate(tmp_path_factory):
         assert (dst[:d0] == 0x5A).all() and (dst[d0 + n:] == 0x5A).all()
         return dst[d0:d0 + n]
     run.write_at = lib_.write_at
+    run.barriers = lib_.barriers
+    run.barriers.restype = C.c_uint64
     return run
 
 
@@ -155,3 +157,15 @@ def test_output_positions_past_32_bits(inflate, stored):
             assert inflate.write_at(start % 2**32, _p(src[s0:]), n, _p(dst[d0:]), stored, 4) == 0
             assert np.array_equal(dst[d0:d0 + n], src[s0:s0 + n])
             assert (dst[:d0] == 0x5A).all() and (dst[d0 + n:] == 0x5A).all(), (start, n)
+
+
+@pytest.mark.parametrize("shape,most", [(1, 300), (2, 450), (3, 650), (4, 650), (5, 800)])
+def test_codes_that_do_not_fall_back_into_step(inflate, shape, most):
+    """Random 7-bit values: codes of one length, whose phase a thread keeps.
+    The threads' starts travel along the segments, a barrier or two each; they
+    do so once, and only over the segments that a step has room for."""
+    raw = np.random.default_rng(1).integers(0, 128, 20000, dtype=np.uint8)
+    c = zlib.compressobj(6, zlib.DEFLATED, -15, 8, zlib.Z_HUFFMAN_ONLY)
+    before = inflate.barriers()
+    assert np.array_equal(inflate(shape, c.compress(raw.tobytes()) + c.flush(), raw.size, 0), raw)
+    assert inflate.barriers() - before <= most
