@@ -82,12 +82,18 @@ __global__ void __launch_bounds__(32 * G) decode_cols_kernel(const uint8_t* __re
 // group decoder's time is a column's serial chain, whatever runs beside it, up
 // to 15 chunks an SM; beyond that it needs fewer instructions a byte, the more
 // so the shorter the columns.  Follow against group, us:
-//   128 KiB chunks   256 MiB 1635 / 2337   512 MiB 3217 / 4172
+//   128 KiB chunks   256 MiB 1635 / 2337   512 MiB 3217 / 4172   1 GiB (55 an SM) 6250 / 7690
 //    64 KiB chunks    64 MiB 331 / 586     512 MiB 2429 / 2637   1 GiB 4827 / 4793
 //    32 KiB chunks    64 MiB 328 / 351     128 MiB 631 / 649     256 MiB 1235 / 1220
 //    16 KiB chunks     8 MiB 64 / 132       16 MiB 111 / 144      32 MiB 202 / 189
 //     4 KiB chunks     1 MiB 21 / 38         2 MiB 32 / 38         4 MiB 52 / 44
 //     1 KiB chunks     1 MiB 29 / 20
+// That is text with copies.  Other columns, the compressed ones above all, are
+// not alike, and the sizes are known only on the device: random bytes in 64 KiB
+// chunks, 512 MiB 1705 / 2546, in 128 KiB, 512 MiB 2840 / 2794, 1 GiB 5620 /
+// 5093; two symbols in 4 KiB, 2 MiB 27 / 19, 16 KiB, 16 MiB 81 / 66, 64 KiB, 512
+// MiB 1420 / 2341; zeros in 64 KiB, 4 MiB 16 / 48, 64 MiB 87 / 71, 512 MiB 632 /
+// 366.
 static bool follow_wins(uint32_t n, uint32_t L) {
     int dev = 0, sms = 148;
     cudaGetDevice(&dev);

@@ -12,11 +12,13 @@
 //              lengths gives the output offsets, literals are stored, and the
 //              matches whose source lies before the first unfinished one are
 //              copied together, 4 bytes a lane and step, until all are done;
+//              after 32 literals, whole groups of literals a lane each;
 //   rows    -- the block stores its part of every row, 16 bytes a thread.
 // The lane-per-column decoders take some 1000 dependent tokens a column and
 // read older history back from the output (15 chunks an SM: more history than
 // the L2 holds): 1.43 ms for 256 MiB in 64 KiB chunks at 39% of the issue
-// slots; this one 1.23 ms at 71%.  Two forms that placed all tokens of a column
+// slots; this one 1.20 ms at 71%; random bytes, all literals, 1.40 and 0.85
+// (a lane per literal throughout: 1.50).  Two forms that placed all tokens of a column
 // first and then resolved its bytes 32 or 128 at a time took 1.34 and 1.28 ms:
 // their tables left room for three blocks an SM instead of five.
 #pragma once
@@ -41,7 +43,7 @@ __host__ __device__ constexpr uint32_t follow_col_smem(uint32_t L) {
 }
 
 template <uint32_t COLS>
-__global__ void __launch_bounds__(COLS * 32) decode_follow_kernel(
+__global__ void __launch_bounds__(COLS * 32, COLS == 8 ? 8 : 12) decode_follow_kernel(
     const uint8_t* __restrict__ data, const uint64_t* __restrict__ blk_off, const uint64_t* __restrict__ col_len,
     const uint8_t* __restrict__ col_map, uint32_t L, uint8_t* __restrict__ out, uint32_t* __restrict__ status) {
     extern __shared__ __align__(16) uint8_t smem[];
@@ -142,7 +144,30 @@ __global__ void __launch_bounds__(COLS * 32) decode_follow_kernel(
         const uint32_t src = o - off;
         uint32_t pend = __ballot_sync(GD_FULL_MASK, live && !lit);
         __syncwarp();
-        while (pend) {
+        const uint32_t end = done + __shfl_sync(GD_FULL_MASK, inc, 31);
+        if (pend == 0) {
+            done = end;
+            // 32 literals: groups of literals as many as follow, up to 32 at a
+            // time, a lane each
+            while ((done & 3u) == 0) {
+                const uint32_t h = g0 + 4u + lane, at = h < ng ? gp[h] : 0u;
+                const bool all = h < ng && s[at] == 0xffu && at + 9u <= len && done + 8u * lane + 8u <= L;
+                const uint32_t run = min(__ffs(~__ballot_sync(GD_FULL_MASK, all)) - 1u, 32u);
+                if (lane < run) {
+                    const uint32_t* w = buf0 + wid * words + ((at + 1u) >> 2);
+                    const uint32_t w1 = w[1], sh = 8u * ((at + 1u) & 3u);
+                    uint32_t* d = out0 + wid * owords + (done >> 2) + 2u * lane;
+                    d[0] = __funnelshift_r(w[0], w1, sh);
+                    d[1] = __funnelshift_r(w1, w[2], sh);
+                }
+                done += 8u * run;
+                g0 += run;
+                if (run < 32u) break;
+            }
+            __syncwarp();
+            continue;
+        }
+        do {
             // everything before the first unfinished match is there
             const uint32_t fo = __shfl_sync(GD_FULL_MASK, o, __ffs(pend) - 1);
             const bool ready = ((pend >> lane) & 1u) && src + min(n, off) <= fo;
@@ -164,8 +189,8 @@ __global__ void __launch_bounds__(COLS * 32) decode_follow_kernel(
             }
             pend &= ~__ballot_sync(GD_FULL_MASK, ready);
             __syncwarp();
-        }
-        done += __shfl_sync(GD_FULL_MASK, inc, 31);
+        } while (pend);
+        done = end;
     }
     if (err == ST_OK && done < L) err = ST_CORRUPT;
     if (err != ST_OK && lane == 0 && status) atomicMax(status + chunk, err);

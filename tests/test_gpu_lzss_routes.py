@@ -21,3 +21,31 @@ def test_number_of_chunks(cuda, chunk, per_sm, over):
     torch.cuda.synchronize()
     assert not job.status().any()
     assert np.array_equal(job.output(), raw)
+
+
+def _runs(rng, n: int, kind: int) -> np.ndarray:
+    """A column of n bytes: repetitions of 1 to 5 bytes of any length one after
+    the other (matches of one offset in a row, begun anywhere in it), or long
+    stretches of literals between short repetitions."""
+    out = []
+    while len(out) < n:
+        unit = rng.integers(0, 256, int(rng.integers(1, 6))).tolist()
+        if kind == 0:
+            out += (unit * 300)[:int(rng.choice([3, 34, 35, 36, 68, 70, 103, 200, 300]))]
+        else:
+            out += rng.integers(0, 256, int(rng.choice([7, 8, 31, 32, 33, 63, 64, 255, 256, 257, 300]))).tolist()
+            out += (unit * 8)[:int(rng.integers(3, 9))]
+    return np.array(out[:n], np.uint8)
+
+
+@pytest.mark.parametrize("chunk", [4096, 16384, 65536, 131072])
+def test_repetitions_and_literals(cuda, chunk):
+    import torch
+    rng = np.random.default_rng(chunk)
+    raw = np.concatenate([np.stack([_runs(rng, chunk // 32, (q + c) % 2 if c else 0).reshape(-1, 4) for q in range(32)], 1)
+                          .reshape(-1) for c in range(4)] + [rng.integers(0, 256, chunk, dtype=np.uint8), np.zeros(chunk, np.uint8)])
+    job = cc.DeviceJob(cc.lzss_encode(raw, chunk))
+    job.launch()
+    torch.cuda.synchronize()
+    assert not job.status().any()
+    assert np.array_equal(job.output(), raw)
