@@ -147,7 +147,11 @@ inline dim3 interleave_grid(uint64_t n_chunks, uint64_t lane_cap) {
 // the candidate lists differ in length, and are serial per lane.)
 
 constexpr uint32_t LZ_WPB = 4;      // columns (warps) per block
-constexpr uint32_t LZ_NB = 512;     // hash buckets of 3-byte keys
+// hash buckets of 3-byte keys; fewer for columns of up to LZ_SHORT bytes, whose
+// time is mostly that of clearing and summing the buckets (1 MiB of text in
+// 128-byte chunks 0.196 ms, 512 buckets 0.575; 1 KiB 44, 94 us; 4 KiB 42, 55)
+constexpr uint32_t LZ_NB = 512, LZ_NB_SHORT = 64, LZ_SHORT = 128;
+__host__ __device__ constexpr uint32_t lz_buckets(uint32_t L) { return L <= LZ_SHORT ? LZ_NB_SHORT : LZ_NB; }
 constexpr uint32_t LZ_HIST = 2048, LZ_MAXM = 34, LZ_MINM = 3;
 constexpr uint32_t LZ_OUT = 256;    // output bytes held back: less than 128, and the next 32 tokens' (37 at most)
 constexpr uint32_t LZ_PAIRS = 256;  // pairs of 32 positions found at once
@@ -155,17 +159,23 @@ constexpr uint32_t LZ_PAIRS = 256;  // pairs of 32 positions found at once
 __host__ __device__ constexpr uint32_t a16(uint32_t x) { return (x + 15u) & ~15u; }
 // column bytes (+64 zero pad) | positions by bucket, also the counts before them | bucket ends | bucket starts (the
 // oldest in the history) | a word per lane | output
-__host__ __device__ constexpr uint32_t lz_pos_bytes(uint32_t L) { return a16(2u * L > 4u * LZ_NB ? 2u * L : 4u * LZ_NB); }
+__host__ __device__ constexpr uint32_t lz_pos_bytes(uint32_t L) {
+    return a16(2u * L > 4u * lz_buckets(L) ? 2u * L : 4u * lz_buckets(L));
+}
 __host__ __device__ constexpr uint32_t lz_warp_smem(uint32_t L) {
-    return a16(L + 64u) + lz_pos_bytes(L) + 4u * LZ_NB + 128u + LZ_OUT;
+    return a16(L + 64u) + lz_pos_bytes(L) + 4u * lz_buckets(L) + 128u + LZ_OUT;
 }
 // the 4 bytes at p
 __device__ __forceinline__ uint32_t lz_word(const uint8_t* d, uint32_t p) {
     const uint32_t* w = reinterpret_cast<const uint32_t*>(d) + (p >> 2);
     return __funnelshift_r(w[0], w[1], 8u * (p & 3u));
 }
-__device__ __forceinline__ uint32_t lz_hash(uint32_t word) { return ((word & 0xffffffu) * 2654435761u) >> 23; }  // 9 bits
+template <uint32_t NB>
+__device__ __forceinline__ uint32_t lz_hash(uint32_t word) {
+    return (((word & 0xffffffu) * 2654435761u) >> 16) * NB >> 16;
+}
 
+template <uint32_t NB>  // lz_buckets of the columns' length
 __global__ void __launch_bounds__(LZ_WPB * 32) lzss_column_kernel(const uint8_t* __restrict__ in, uint64_t n_bytes,
                                                                   uint64_t chunk_size, uint32_t n_cols,
                                                                   uint8_t* __restrict__ scratch, uint32_t cap,
@@ -180,8 +190,8 @@ __global__ void __launch_bounds__(LZ_WPB * 32) lzss_column_kernel(const uint8_t*
     uint16_t* pos = reinterpret_cast<uint16_t*>(d + a16(L + 64u));
     uint32_t* cnt = reinterpret_cast<uint32_t*>(pos);
     uint16_t* end = reinterpret_cast<uint16_t*>(reinterpret_cast<uint8_t*>(pos) + lz_pos_bytes(L));
-    uint16_t* start = end + LZ_NB;
-    uint32_t* area = reinterpret_cast<uint32_t*>(start + LZ_NB);
+    uint16_t* start = end + NB;
+    uint32_t* area = reinterpret_cast<uint32_t*>(start + NB);
     uint8_t* out = reinterpret_cast<uint8_t*>(area + 32);
     const bool aged = L > LZ_HIST;  // candidates can leave the history
 
@@ -200,16 +210,16 @@ __global__ void __launch_bounds__(LZ_WPB * 32) lzss_column_kernel(const uint8_t*
         reinterpret_cast<uint32_t*>(d)[k] = w;
     }
     for (uint32_t i = L / 4u + lane; i < L / 4u + 16u; i += 32) reinterpret_cast<uint32_t*>(d)[i] = 0;
-    for (uint32_t b = lane; b < LZ_NB; b += 32) cnt[b] = 0;
+    for (uint32_t b = lane; b < NB; b += 32) cnt[b] = 0;
     __syncwarp();
 
     // ---- where each bucket of the positions with a full key (p + 2 < L)
     // starts; not the first, which is never a source ----
     const uint32_t np = L - 2u;
-    for (uint32_t p = 1u + lane; p < np; p += 32) atomicAdd(&cnt[lz_hash(lz_word(d, p))], 1u);
+    for (uint32_t p = 1u + lane; p < np; p += 32) atomicAdd(&cnt[lz_hash<NB>(lz_word(d, p))], 1u);
     __syncwarp();
     {
-        constexpr uint32_t PER = LZ_NB / 32u;
+        constexpr uint32_t PER = NB / 32u;
         uint32_t v[PER], sum = 0;
 #pragma unroll
         for (uint32_t i = 0; i < PER; ++i) {
@@ -254,7 +264,7 @@ __global__ void __launch_bounds__(LZ_WPB * 32) lzss_column_kernel(const uint8_t*
         // ---- the next 32 positions into their buckets ----
         const uint32_t p = w0 + lane, w = lz_word(d, p);
         const bool keyed = p >= 1u && p < np;
-        const uint32_t h = keyed ? lz_hash(w) : LZ_NB + lane;
+        const uint32_t h = keyed ? lz_hash<NB>(w) : NB + lane;
         const uint32_t peers = __match_any_sync(GD_FULL_MASK, h);
         uint32_t at = 0, first = 0;
         if (keyed) {
@@ -530,9 +540,10 @@ extern "C" gd_status_t gd_lzss_encode_device(const uint8_t* d_in, uint64_t n_byt
     const uint32_t L = (uint32_t)(chunk_size / 32u);
     const uint32_t wsm = lz_warp_smem(L);
     cudaStream_t s = (cudaStream_t)stream;
-    cudaFuncSetAttribute(lzss_column_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, LZ_WPB * wsm);
+    auto kern = lz_buckets(L) == LZ_NB ? lzss_column_kernel<LZ_NB> : lzss_column_kernel<LZ_NB_SHORT>;
+    cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, LZ_WPB * wsm);
     const uint32_t ncol = (uint32_t)(nc * 32u);
-    lzss_column_kernel<<<(ncol + LZ_WPB - 1) / LZ_WPB, LZ_WPB * 32, LZ_WPB * wsm, s>>>(
+    kern<<<(ncol + LZ_WPB - 1) / LZ_WPB, LZ_WPB * 32, LZ_WPB * wsm, s>>>(
         d_in, n_bytes, chunk_size, ncol, d_scratch, (uint32_t)cap, raw_len, wsm);
     lzss_rank_kernel<<<(uint32_t)((nc + NT / 32 - 1) / (NT / 32)), NT, 0, s>>>(raw_len, (uint32_t)nc, d_col_len,
                                                                               d_col_map, d_blk_off + 1, d_status);

@@ -22,7 +22,10 @@ extern "C" int lzss_columns(const uint8_t* in, uint64_t chunk_size, uint32_t fir
     for (uint32_t b = first / LZ_WPB; b < n_cols / LZ_WPB; ++b) {
         memset(smem, 0, sizeof smem);
         if (!simt::run(32 * LZ_WPB, b, 32 / LZ_WPB, simt::schedule(32 * LZ_WPB, kind), [&] {
-                lzss_column_kernel(in, chunk_size, chunk_size, 32, scratch, cap, raw_len, wsm);
+                if (lz_buckets((uint32_t)(chunk_size / 32)) == LZ_NB)
+                    lzss_column_kernel<LZ_NB>(in, chunk_size, chunk_size, 32, scratch, cap, raw_len, wsm);
+                else
+                    lzss_column_kernel<LZ_NB_SHORT>(in, chunk_size, chunk_size, 32, scratch, cap, raw_len, wsm);
             }))
             return 1;
     }

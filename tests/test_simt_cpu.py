@@ -21,7 +21,7 @@ SCHEDULES = [0, 1, 2, 3, 4, 11, 12, 100, 101]  # see simt::schedule
 
 
 def _compile(src: Path, out: Path, *flags) -> C.CDLL:
-    cmd = ["g++", "-std=c++20", "-O1", "-w", "-shared", "-fPIC", "-I", str(SIMT), "-I",
+    cmd = ["g++", "-std=c++20", "-O1", "-w", "-fno-extern-tls-init", "-shared", "-fPIC", "-I", str(SIMT), "-I",
            str(ROOT / "compression_b200" / "csrc"), *flags, str(src), "-o", str(out)]
     r = subprocess.run(cmd, capture_output=True, text=True)
     assert r.returncode == 0, r.stderr
