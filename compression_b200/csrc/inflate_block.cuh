@@ -53,7 +53,8 @@ constexpr uint32_t LBITS = 10, DBITS = 8;  // primary lookup bits
 // Bits per segment: 8 above a multiple of 64, so that threads that sit at the
 // same place in their segments read 32 different shared-memory banks (256
 // bits would put eight threads of a warp on each of four banks).
-constexpr uint32_t KSEG = 264, KQ = KSEG / 4;
+// Fewer where the rest of the stream does not fill the block's threads.
+constexpr uint32_t KSEG = 264, KSEG_MID = 136, KSEG_LOW = 72;
 
 // Code-length code order (RFC 1951 3.2.7).
 __device__ __constant__ uint8_t CLEN_ORDER[19] = {16, 17, 18, 0, 8, 7, 9, 6, 10, 5, 11, 4, 12, 3, 13, 2, 14, 1, 15};
@@ -100,7 +101,6 @@ struct alignas(16) Smem {
     uint32_t exits[NT];
     uint32_t red[NW + 1];       // scans
     uint32_t evw[NW];
-    uint32_t cnt[16];           // build_code
     uint32_t use_n, use_bit, use_ev;      // of the last thread taken from a step
     uint32_t take, take_T, take_c, bad, n_big;  // of a placement
     alignas(4) uint8_t lens[320];  // code lengths of a block
@@ -156,52 +156,48 @@ __device__ __forceinline__ uint32_t long_code(const Code<BITS, NS>& h, uint32_t 
     return make_entry(tk, h.sym[(int32_t)(c >> (15 - L)) + h.delta[L]], L);
 }
 
-// Build `h` from code lengths lens[0..n) for table kind tk: warp 0 sorts the
-// symbols by length (stable, 32 a round) and finds the canonical limits, then
-// every table index finds its own code.  Returns false (on every thread) for
-// an over-subscribed code.  Called by the whole block.
-template <uint32_t BITS, uint32_t NS>
-static __device__ bool build_code(Code<BITS, NS>& h, const uint8_t* lens, uint32_t n, uint32_t* cnt, uint32_t tk) {
-    const uint32_t lane = lane_id(), lt = (1u << lane) - 1u;
+// Build `h` from code lengths lens[0..n) for table kind tk: the warps count
+// the lengths of 32 symbols each (tab: 16 words for every 32 symbols), warp 0
+// finds the canonical limits, the warps sort their symbols by length (stable),
+// then every table index finds its own code.  Returns false (on every thread)
+// for an over-subscribed code.  Called by the whole block (NW warps).
+template <int NW, uint32_t BITS, uint32_t NS>
+static __device__ bool build_code(Code<BITS, NS>& h, const uint8_t* lens, uint32_t n, uint32_t* tab, uint32_t tk) {
+    const uint32_t lane = lane_id(), wid = threadIdx.x >> 5, groups = (n + 31u) / 32u;
+    for (uint32_t i = threadIdx.x; i < 16u * groups; i += 32u * NW) tab[i] = 0;
+    __syncthreads();
+    for (uint32_t g = wid; g < groups; g += NW) {
+        const uint32_t i = 32u * g + lane, L = i < n ? lens[i] : 0u;
+        const uint32_t peers = __match_any_sync(GD_FULL_MASK, L);
+        if ((peers & ((1u << lane) - 1u)) == 0) tab[16u * g + L] = __popc(peers);
+    }
+    __syncthreads();
     bool ok = true;
-    if (threadIdx.x < 32) {
-        if (lane < 16) cnt[lane] = 0;
-        __syncwarp();
-        for (uint32_t b = 0; b < n; b += 32) {
-            const uint32_t L = b + lane < n ? lens[b + lane] : 0u;
-            const uint32_t peers = __match_any_sync(GD_FULL_MASK, L);
-            if ((peers & lt) == 0) cnt[L] += __popc(peers);
-            __syncwarp();
-        }
-        // lane L: first code and first index of length L
-        uint32_t code = 0, idx = 0;
-        for (uint32_t l = 1; l < 16; ++l) {
-            const uint32_t k = cnt[l];
-            if (lane >= l) {
-                const uint32_t prev = l > 1 ? cnt[l - 1] : 0u;
-                code = (code + prev) << 1;
-                idx += prev;
+    if (wid == 0) {
+        // lane L: codes of length L, and where the next length's start
+        const bool length = lane >= 1u && lane < 16u;
+        uint32_t k = 0;
+        for (uint32_t g = 0; g < groups; ++g) k += length ? tab[16u * g + lane] : 0u;
+        const uint32_t share = length ? k << (15u - lane) : 0u, lim = warp_incl_scan(share);
+        uint32_t idx = warp_incl_scan(k) - k;
+        if (length) {
+            ok = lim <= 32768u;
+            h.lim[lane] = (uint16_t)min(lim, 32768u);
+            h.delta[lane] = (int16_t)((int32_t)idx - (int32_t)((lim - share) >> (15u - lane)));
+            for (uint32_t g = 0; g < groups; ++g) {
+                const uint32_t c = tab[16u * g + lane];
+                tab[16u * g + lane] = idx;
+                idx += c;
             }
-            if (lane == l) {
-                ok = code + k <= (1u << l);
-                h.lim[l] = (uint16_t)min((code + k) << (15u - l), 32768u);
-                h.delta[l] = (int16_t)((int32_t)idx - (int32_t)code);
-            }
-        }
-        __syncwarp();
-        if (lane < 16) cnt[lane] = idx;  // sort cursors (length 0 is not used)
-        __syncwarp();
-        for (uint32_t b = 0; b < n; b += 32) {
-            const uint32_t L = b + lane < n ? lens[b + lane] : 0u;
-            const uint32_t peers = __match_any_sync(GD_FULL_MASK, L);
-            const uint32_t at = cnt[L] + __popc(peers & lt);
-            __syncwarp();
-            if (L) h.sym[at] = (uint16_t)(b + lane);
-            if ((peers & lt) == 0) cnt[L] = at + __popc(peers);
-            __syncwarp();
         }
     }
     if (__syncthreads_or(!ok)) return false;
+    for (uint32_t g = wid; g < groups; g += NW) {
+        const uint32_t i = 32u * g + lane, L = i < n ? lens[i] : 0u;
+        const uint32_t peers = __match_any_sync(GD_FULL_MASK, L);
+        if (L) h.sym[tab[16u * g + L] + __popc(peers & ((1u << lane) - 1u))] = (uint16_t)i;
+    }
+    __syncthreads();
     uint32_t lim[BITS + 1];
 #pragma unroll
     for (uint32_t l = 1; l <= BITS; ++l) lim[l] = h.lim[l];
@@ -609,7 +605,7 @@ static __device__ __forceinline__ uint32_t stream_block(const uint8_t* __restric
 
     Writer<SmemT> wr(S, dst);
     uint32_t bfinal = 0;
-    uint32_t lim = NT;  // threads that decode a step's segments
+    uint32_t lim = NT, kseg = KSEG;  // threads that decode a step's segments, and their bits
     while (err == ST_OK && !bfinal) {
         // ---- block header (every thread reads the same bits) ----
         stage();
@@ -665,7 +661,7 @@ static __device__ __forceinline__ uint32_t stream_block(const uint8_t* __restric
             }
             bp += 3u * ncl;
             __syncthreads();
-            if (!build_code(S.dist, S.lens, 19, S.cnt, TK_PLAIN)) {
+            if (!build_code<NW>(S.dist, S.lens, 19, S.sym, TK_PLAIN)) {
                 err = ST_CORRUPT;
                 break;
             }
@@ -731,8 +727,8 @@ static __device__ __forceinline__ uint32_t stream_block(const uint8_t* __restric
         }
         __syncthreads();
         if (S.lens[256] == 0 ||  // no end-of-block code
-            !build_code(S.lit, S.lens, nlen, S.cnt, TK_LIT) ||
-            !build_code(S.dist, S.lens + nlen, ndist, S.cnt, TK_DIST)) {
+            !build_code<NW>(S.lit, S.lens, nlen, S.sym, TK_LIT) ||
+            !build_code<NW>(S.dist, S.lens + nlen, ndist, S.sym, TK_DIST)) {
             err = ST_CORRUPT;
             break;
         }
@@ -747,7 +743,11 @@ static __device__ __forceinline__ uint32_t stream_block(const uint8_t* __restric
             // positions below count bits from b0
             const uint32_t p0 = (uint32_t)(bp - b0);
             const uint32_t avail = (uint32_t)min((unsigned long long)(bend - b0), 0x40000000ull);
-            const uint32_t seg = p0 + tid * KSEG;
+            if (avail - p0 <= NT * KSEG_MID && kseg != KSEG_LOW) {
+                kseg = avail - p0 <= NT * KSEG_LOW ? KSEG_LOW : KSEG_MID;
+                lim = NT;
+            }
+            const uint32_t seg = p0 + tid * kseg;
             uint32_t s = min(seg, avail), pos = s;  // where this thread starts, and leaves its segment
             uint32_t n = 0;                         // symbols
             uint32_t ev = 0, evn = 0, evs = 0;      // first special one (E_EOB / E_BAD): index, start
@@ -759,7 +759,7 @@ static __device__ __forceinline__ uint32_t stream_block(const uint8_t* __restric
                     const uint32_t k = S.sym[j * NT + tid];
                     if ((k & 63u) != s - seg) continue;
                     n = (k >> 6) & 511u;
-                    pos = seg + KSEG + ((k >> 15) & 63u);
+                    pos = seg + kseg + ((k >> 15) & 63u);
                     evn = (k >> 21) & 511u;
                     ev = k >> 30 << 1;
                     cps = false;
@@ -774,7 +774,7 @@ static __device__ __forceinline__ uint32_t stream_block(const uint8_t* __restric
                     pos = s;
                     n = ev = 0;
                     for (uint32_t q = 0; q < 4; ++q) {
-                        const uint32_t to = min(seg + (q + 1) * KQ, avail);
+                        const uint32_t to = min(seg + (q + 1) * (kseg / 4u), avail);
                         uint32_t at = pos;
                         while (pos < to) {
                             uint32_t word;
@@ -813,9 +813,9 @@ static __device__ __forceinline__ uint32_t stream_block(const uint8_t* __restric
                         S.cp[q][tid] = here | (n << 16);
                     }
                     cps = true;
-                    if (s - seg < 64u && pos >= seg + KSEG) {
+                    if (s - seg < 64u && pos >= seg + kseg) {
                         S.sym[(kept % KEEP) * NT + tid] =
-                            (s - seg) | (n << 6) | ((pos - seg - KSEG) << 15) | (ev ? evn << 21 | ev << 29 : 0u);
+                            (s - seg) | (n << 6) | ((pos - seg - kseg) << 15) | (ev ? evn << 21 | ev << 29 : 0u);
                         ++kept;
                     }
                 }
