@@ -380,10 +380,11 @@ def test_lzss_token_shapes(cuda, knob, chunk):
     assert np.array_equal(out, ref)
 
 
-@pytest.mark.parametrize("variant", [0, 1, 2, 3, 4, 5, 6, 7, 8, 9, 10, 11, 12, 13, 14])
+@pytest.mark.parametrize("variant", [0, 1, 2, 3, 4, 6, 12, 13])
 def test_inflate_variants(cuda, variant):
-    """Every inflate kernel shape on streams of mixed size with dynamic,
-    fixed-Huffman and stored blocks, against zlib."""
+    """Every inflate kernel shape (1 - 4 a block per stream, 6 and 12 a warp
+    pair), and the choice among them (0, or a value of no shape), on streams of
+    mixed size with dynamic, fixed-Huffman and stored blocks, against zlib."""
     import compression_b200.autotune as at
     raw = cc.gen_markov_copy(11, 3 << 20, 32768)
     sizes = cc.loguniform_sizes(12, 40, 1024, 256 * 1024, raw.size)
