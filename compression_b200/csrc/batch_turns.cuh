@@ -71,18 +71,19 @@ __device__ __forceinline__ void run_turns(uint32_t n, const uint32_t* __restrict
                 bool defl = false, soon = false;
                 uint32_t ti = first;
                 first = NONE;
-                if (!dynamic) {
-                    // a warp goes on to its next Deflate task, or its end
-                    do {
-                        ti = entry(at);
-                        at += W;
-                    } while (ti == BAD);
-                    defl = ti != NONE && deflate(ti);
-                } else if (ti == NONE) {
+                if (ti == NONE) {
                     uint32_t stop = 0;
                     if (lane == 0) stop = *(volatile uint32_t*)&s_stop;
                     if (__shfl_sync(GD_FULL_MASK, stop, 0)) break;
-                    ti = pop(defl, soon);
+                    if (dynamic) {
+                        ti = pop(defl, soon);
+                    } else {
+                        do {
+                            ti = entry(at);
+                            at += W;
+                        } while (ti == BAD);
+                        defl = ti != NONE && deflate(ti);
+                    }
                 }
                 if (ti != NONE && !defl) warp_task(ti);
                 const bool leave = ti == NONE || defl || soon;
@@ -90,7 +91,8 @@ __device__ __forceinline__ void run_turns(uint32_t n, const uint32_t* __restrict
                     if (ti == NONE && dynamic) s_end = 1;
                     if (soon) s_soon = 1;
                     if (defl) s_list[atomicAdd(&s_nd, 1u)] = ti;
-                    if (leave) *(volatile uint32_t*)&s_stop = 1;
+                    // statically, a warp at its end leaves the others going
+                    if (leave && (dynamic || defl)) *(volatile uint32_t*)&s_stop = 1;
                 }
                 if (leave) break;
                 __syncwarp();
