@@ -9,16 +9,19 @@
 // single kernel can run them all.  Tasks come from a global atomic counter
 // over an order array (dynamic: with tasks sorted longest-first this is LPT
 // list scheduling) or from the static mapping task i -> warp i mod W.
-// In a dynamic launch every warp takes its own tasks, until one takes a
-// Deflate task or sees one ahead (31 samples of the part of the queue that the
+// Every warp takes its own tasks, until one takes a Deflate task or, in a
+// dynamic launch, sees one ahead (31 samples of the part of the queue that the
 // blocks will take next): then the block's warps finish what they have and the
-// Deflate stream is decoded.  While Deflate tasks lie ahead the block takes one
-// task at a time, so that no block collects several of the largest tasks and
-// runs them one after another; a task that is no Deflate task after all lets
-// all warps go on.
+// Deflate stream is decoded (batch_turns.cuh).  While Deflate tasks lie ahead in
+// the queue the block takes one task at a time, so that no block collects
+// several of the largest tasks and runs them one after another; a task that is
+// no Deflate task after all lets all warps go on.
 // A Deflate stream on one warp (one lane decoding) set the makespan: 256 MiB
-// in 1024 items, the largest stream 1.7 MB, longest first: 16.1 -> 1.9 ms; with
-// four warps a block and stream 3.0 ms (the largest stream alone takes 2.9).
+// in 1024 items, the largest stream 1.7 MB, longest first: 16.2 -> 1.73 ms (with
+// four warps a block and stream half as much again).  What it costs: warps wait
+// for one another where short Deflate tasks lie among others (64 MiB of items
+// of 2 to 64 KiB 0.99 -> 1.16 ms), and thousands of tiny ones take the blocks one
+// by one (20,000 of 0.2 to 2 KB 1.76 -> 2.19 ms).
 // Per-task %globaltimer start/end stamps (optional) are the measurements the
 // learned cost model trains on.
 #include "batch_turns.cuh"

@@ -159,11 +159,11 @@ gd_status_t launch_block(const Chunks& ch, uint32_t n, int zlib_hdr, const uint3
 // a 32 / 4 KiB window, whose hand-off wait the test knobs bound; any other
 // value = by the number of streams:
 //   up to one a SM: 16 warps and the largest window and placement (39 streams
-//   of 128 KiB: 0.107 ms; 8 warps 0.165; the warp pair 1.05);
+//   of 128 KiB: 0.099 ms; 8 warps 0.159; the warp pair 1.00);
 //   up to two a SM: 8 warps, two blocks a SM;
 //   more: 8 warps, three blocks a SM (2048 streams of 4 KiB to 700 KiB,
-//   256 MiB: 1.04 ms; two blocks with twice the placement 1.10; 4 warps
-//   1.47; 16 warps 1.16; the warp pair 5.09).
+//   256 MiB: 0.96 ms; two blocks with twice the placement 1.03; four with half
+//   the window 0.99; 16 warps 1.25; the warp pair 5.1).
 template <class Chunks>
 gd_status_t launch_inflate(const Chunks& ch, uint32_t n, int zlib_hdr, const uint32_t* order, cudaStream_t s) {
     int v = gd_tune_get(GD_TUNE_INFLATE_VARIANT);

@@ -53,7 +53,9 @@ constexpr uint32_t LBITS = 10, DBITS = 8;  // primary lookup bits
 // Bits per segment: 8 above a multiple of 64, so that threads that sit at the
 // same place in their segments read 32 different shared-memory banks (256
 // bits would put eight threads of a warp on each of four banks).
-// Fewer where the rest of the stream does not fill the block's threads.
+// Fewer where the rest of the stream does not fill the block's threads: a
+// short stream's time is that of a few threads' chains (16,384 streams of 1 KiB
+// of text 1.43 ms at 264 bits, 1.20 at 72).
 constexpr uint32_t KSEG = 264, KSEG_MID = 136, KSEG_LOW = 72;
 
 // Code-length code order (RFC 1951 3.2.7).

@@ -226,9 +226,9 @@ typedef struct gd_task {
 /*
  * Decode n_tasks tasks in one persistent launch (blocks_per_sm x SMs blocks
  * of 8 warps, 4 for very long lanes; 0 = as many as fit).  dynamic = 1: warps take tasks in the
- * order d_order[0..n) (NULL = identity) from a work queue whose counter is
+ * order d_order[0..n) (NULL = identity; entries >= n_tasks are passed over) from a work queue whose counter is
  * d_counter (one uint32 of caller scratch, zeroed by this call); dynamic = 0:
- * task d_order[i] runs on warp i mod W.  max_lane_bytes bounds col_len of
+ * task d_order[i] runs on warp i mod W, a Deflate task on that warp's whole block.  max_lane_bytes bounds col_len of
  * RLE tasks.  d_status[n] (task index order) and optional d_timing[2n]
  * (%globaltimer ns at each task's start and end) are written per task.
  */
