@@ -148,9 +148,10 @@ inline dim3 interleave_grid(uint64_t n_chunks, uint64_t lane_cap) {
 
 constexpr uint32_t LZ_WPB = 4;      // columns (warps) per block
 // hash buckets of 3-byte keys; fewer for columns of up to LZ_SHORT bytes, whose
-// time is mostly that of clearing and summing the buckets (1 MiB of text in
-// 128-byte chunks 0.196 ms, 512 buckets 0.575; 1 KiB 44, 94 us; 4 KiB 42, 55)
-constexpr uint32_t LZ_NB = 512, LZ_NB_SHORT = 64, LZ_SHORT = 128;
+// time is mostly that of clearing and summing the buckets (4 MiB in 8 KiB chunks:
+// zeros 0.102 ms, 512 buckets 0.123, 64 0.101; text 0.098, 0.115, 0.106; 1 MiB of
+// text in 512-byte chunks 0.064, 0.159, 0.063)
+constexpr uint32_t LZ_NB = 512, LZ_NB_SHORT = 128, LZ_SHORT = 256;
 __host__ __device__ constexpr uint32_t lz_buckets(uint32_t L) { return L <= LZ_SHORT ? LZ_NB_SHORT : LZ_NB; }
 constexpr uint32_t LZ_HIST = 2048, LZ_MAXM = 34, LZ_MINM = 3;
 constexpr uint32_t LZ_OUT = 256;    // output bytes held back: less than 128, and the next 32 tokens' (37 at most)

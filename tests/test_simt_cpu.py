@@ -125,7 +125,7 @@ def lzss_columns(tmp_path_factory):
     return _compile(SIMT / "lzss_columns.cpp", tmp / "lzss.so", f'-DLZSS_COLUMNS="{tmp / "cols.inc"}"').lzss_columns
 
 
-@pytest.mark.parametrize("chunk", [1024, 65536, 131072])
+@pytest.mark.parametrize("chunk", [1024, 8192, 8320, 65536, 131072])
 @pytest.mark.parametrize("kind", [0, 1, 2, 11])
 def test_lzss_columns_match_the_host_encoder(lzss_columns, chunk, kind):
     rng = np.random.default_rng(chunk)
