@@ -5,9 +5,9 @@
 // rlev2::compress_gpu_transpose, include/rlev2/encoder_trans.h:428-537),
 // producing the same bytes as the host encoders (gd_encode.cpp, lane_enc.h).
 // Launches on one stream:
-//   1. the lane streams, a warp each (rlev1_enc.cuh, rlev2_enc.cuh), into
-//      scratch slots; then a warp per chunk sums the padded word counts into
-//      the chunk's block size;
+//   1. the lane streams, a warp each (rlev1_enc.cuh, rlev2_enc.cuh) or a thread
+//      each (rle_thread_enc.cuh), into scratch slots; then a warp per chunk sums
+//      the padded word counts into the chunk's block size;
 //   2. offsets_kernel: one block turns the block sizes into blk_off;
 //   3. interleave_kernel: row k = one word of every lane longer than 4k bytes,
 //      in lane order, through the same segment table the decoders read with
@@ -16,6 +16,7 @@
 #include "gd_common.cuh"
 #include "interleave.cuh"
 #include "lane_enc.h"
+#include "rle_thread_enc.cuh"
 #include "rlev1_enc.cuh"
 #include "rlev2_enc.cuh"
 
@@ -448,6 +449,36 @@ inline uint64_t rlev2_lane_cap(uint64_t chunk_size) {
     return (nv * 11u + 64u + 3u) & ~3ull;
 }
 
+// Lane streams of n values by a thread each where that is the faster: its time
+// grows with n and, up to a chip full of them, hardly with their number; the warp
+// encoders' grows with the tokens.  Time by threads over time by warps, RLE v1 of
+// 4-byte values:
+//    n    lanes: 8 K  32 K  128 K  512 K   (runs and literals alternating)
+//     8          0.42  0.45   0.41   0.42
+//    16          0.88  0.62   0.50   0.47
+//    32          1.28  0.97   0.67   0.66
+//    64          1.95  1.46   0.99   0.88
+//   128          2.39  1.44   1.06   1.14
+//   512          4.4   2.2    1.4    1.7
+//  1024          8.4   3.4    2.3    2.3
+// and of runs of 8 equal values, which are a token each, n = 128 0.94, 0.39, 0.22,
+// 0.21, n = 1024 1.85, 0.61, 0.25, 0.22; RLE v2 n = 16 1.82, 1.07, 0.89, 0.78, n =
+// 1024 18.8, 7.4, 6.4, of runs n = 32 1.33, 0.89, 0.78, 0.58, n = 1024 1.75, 0.64,
+// 0.54.  So short lanes go by the sizes, and in columns of over 16,384 lanes
+// (n < 512: as many) a sample tells: an end of a run for every 32 values (RLE v2:
+// 14).  It and the launch that finds nothing to do take 6 to 8 us, which smaller
+// columns would feel (64 MiB in 128 KiB chunks 0.224 ms); there runs of 8 take
+// 0.50 ms by warps, 0.30 by threads.
+inline ThreadRule rlev1_by_thread(uint64_t lanes, uint64_t n) {
+    const bool all = n < 16 || (n < 32 && lanes >= 8192) || (n < 64 && lanes >= 32768) || (n < 128 && lanes >= 65536) ||
+                     (n < 256 && lanes >= 131072);
+    return {all, !all && (lanes > 16384 || (n < 512 && lanes >= 16384)) ? SAMPLE : 0u};
+}
+inline ThreadRule rlev2_by_thread(uint64_t lanes, uint64_t n) {
+    const bool all = n < 4 || (n < 8 && lanes >= 8192) || (n < 16 && lanes >= 16384) || (n < 32 && lanes >= 32768);
+    return {all, !all && (lanes > 16384 || (n < 512 && lanes >= 16384)) ? SAMPLE * 9u / 4u : 0u};
+}
+
 // blk_off from the block sizes, then the container.
 inline gd_status_t finish(uint64_t nc, const uint8_t* d_scratch, uint64_t lane_cap, uint8_t* d_data,
                           uint64_t* d_blk_off, const uint64_t* d_col_len, const uint8_t* d_col_map, cudaStream_t s) {
@@ -487,10 +518,26 @@ extern "C" gd_status_t gd_rlev1_encode_device(const uint8_t* d_in, uint64_t n_by
     const uint32_t wil = comp_col_len / elem_bytes;
     cudaStream_t s = (cudaStream_t)stream;
     const uint64_t nc = (n_bytes + chunk_size - 1) / chunk_size;
-    auto kern = elem_bytes == 4 ? rlev1_encode_kernel<uint32_t> : rlev1_encode_kernel<uint64_t>;
-    kern<<<(uint32_t)((nc * 32u + V1_WPB - 1) / V1_WPB), V1_WPB * 32, 0, s>>>(d_in, n_bytes, nc * 32u, chunk_size, wil,
-                                                                              d_scratch, (uint32_t)cap, d_col_len);
-    lane_sizes_kernel<<<(uint32_t)((nc + 3) / 4), 128, 0, s>>>((uint32_t)nc, d_col_len, d_blk_off + 1, d_status);
+    auto go = [&](auto value) {
+        using T = decltype(value);
+        const ThreadRule by = rlev1_by_thread(nc * 32u, chunk_size / 32u / sizeof(T));
+        uint64_t* runs = by.ends ? d_blk_off : nullptr;  // until the offsets are there
+        if (runs)
+            sample_runs_kernel<GD_CODEC_RLEV1, T>
+                <<<1, 1024, 0, s>>>(reinterpret_cast<const T*>(d_in), n_bytes / sizeof(T), by.ends, runs);
+        if (by.all || runs)
+            thread_encode_kernel<GD_CODEC_RLEV1, T><<<(uint32_t)((nc + 3) / 4), THREAD_NT, 0, s>>>(
+                d_in, n_bytes, (uint32_t)nc, chunk_size, wil, d_scratch, (uint32_t)cap, d_col_len, runs, d_blk_off + 1,
+                d_status);
+        if (!by.all) {
+            rlev1_encode_kernel<T><<<(uint32_t)((nc * 32u + V1_WPB - 1) / V1_WPB), V1_WPB * 32, 0, s>>>(
+                d_in, n_bytes, nc * 32u, chunk_size, wil, d_scratch, (uint32_t)cap, d_col_len, runs);
+            lane_sizes_kernel<<<(uint32_t)((nc + 3) / 4), 128, 0, s>>>((uint32_t)nc, d_col_len, d_blk_off + 1,
+                                                                       d_status);
+        }
+    };
+    if (elem_bytes == 4) go(uint32_t{});
+    else go(uint64_t{});
     return finish(nc, d_scratch, cap, d_data, d_blk_off, d_col_len, nullptr, s);
 }
 
@@ -513,9 +560,20 @@ extern "C" gd_status_t gd_rlev2_encode_device(const uint8_t* d_in, uint64_t n_by
     if ((n_bytes + chunk_size - 1) / chunk_size > 0xffffffffull) return GD_ERR_UNSUPPORTED;
     const uint64_t nc = (n_bytes + chunk_size - 1) / chunk_size, cap = rlev2_lane_cap(chunk_size);
     cudaStream_t s = (cudaStream_t)stream;
-    rlev2_encode_kernel<<<(uint32_t)((nc * 32u + V2_WPB - 1) / V2_WPB), V2_WPB * 32, 0, s>>>(
-        d_in, n_bytes, nc * 32u, chunk_size, read_unit, d_scratch, (uint32_t)cap, d_col_len);
-    lane_sizes_kernel<<<(uint32_t)((nc + 3) / 4), 128, 0, s>>>((uint32_t)nc, d_col_len, d_blk_off + 1, d_status);
+    const ThreadRule by = rlev2_by_thread(nc * 32u, chunk_size / 256u);
+    uint64_t* runs = by.ends ? d_blk_off : nullptr;  // until the offsets are there
+    if (runs)
+        sample_runs_kernel<GD_CODEC_RLEV2, int64_t>
+            <<<1, 1024, 0, s>>>(reinterpret_cast<const int64_t*>(d_in), n_bytes / 8u, by.ends, runs);
+    if (by.all || runs)
+        thread_encode_kernel<GD_CODEC_RLEV2, int64_t><<<(uint32_t)((nc + 3) / 4), THREAD_NT, 0, s>>>(
+            d_in, n_bytes, (uint32_t)nc, chunk_size, read_unit, d_scratch, (uint32_t)cap, d_col_len, runs, d_blk_off + 1,
+            d_status);
+    if (!by.all) {
+        rlev2_encode_kernel<<<(uint32_t)((nc * 32u + V2_WPB - 1) / V2_WPB), V2_WPB * 32, 0, s>>>(
+            d_in, n_bytes, nc * 32u, chunk_size, read_unit, d_scratch, (uint32_t)cap, d_col_len, runs);
+        lane_sizes_kernel<<<(uint32_t)((nc + 3) / 4), 128, 0, s>>>((uint32_t)nc, d_col_len, d_blk_off + 1, d_status);
+    }
     return finish(nc, d_scratch, cap, d_data, d_blk_off, d_col_len, nullptr, s);
 }
 

@@ -40,16 +40,18 @@ __device__ __forceinline__ void v1_put_varint(T v, uint32_t nb, uint8_t* out) {
 }
 
 // A warp per lane stream; col_len gets the stream's bytes, all ones if they
-// outgrew the slot (lane_sizes_kernel turns that into a status).
+// outgrew the slot (lane_sizes_kernel turns that into a status).  skip (or
+// null): nothing to do if it is not 0.
 template <typename T>
 __global__ void __launch_bounds__(V1_WPB * 32) rlev1_encode_kernel(const uint8_t* __restrict__ in, uint64_t n_bytes,
                                                                    uint64_t n_lanes, uint64_t chunk_size, uint32_t wil,
                                                                    uint8_t* __restrict__ scratch, uint32_t lane_cap,
-                                                                   uint64_t* __restrict__ col_len) {
+                                                                   uint64_t* __restrict__ col_len,
+                                                                   const uint64_t* __restrict__ skip) {
     __shared__ V1Warp<T> smem[V1_WPB];
     const uint32_t lane = lane_id(), wid = threadIdx.x >> 5;
     const uint64_t id = (uint64_t)blockIdx.x * V1_WPB + wid;  // 32 * chunk + lane stream
-    if (id >= n_lanes) return;                                 // warp-uniform
+    if (id >= n_lanes || (skip && *skip)) return;      // warp-uniform
     V1Warp<T>& S = smem[wid];
     const uint64_t cb = (id >> 5) * chunk_size;
     const uint64_t avail =

@@ -301,15 +301,17 @@ __device__ __forceinline__ uint32_t v2_var_run(V2Warp& S, uint32_t i, uint32_t m
 }
 
 // A warp per lane stream; col_len gets the stream's bytes, all ones if they
-// outgrew the slot (lane_sizes_kernel turns that into a status).
+// outgrew the slot (lane_sizes_kernel turns that into a status).  skip (or
+// null): nothing to do if it is not 0.
 __global__ void __launch_bounds__(V2_WPB * 32) rlev2_encode_kernel(const uint8_t* __restrict__ in, uint64_t n_bytes,
                                                                    uint64_t n_lanes, uint64_t chunk_size,
                                                                    uint32_t read_unit, uint8_t* __restrict__ scratch,
-                                                                   uint32_t lane_cap, uint64_t* __restrict__ col_len) {
+                                                                   uint32_t lane_cap, uint64_t* __restrict__ col_len,
+                                                                   const uint64_t* __restrict__ skip) {
     __shared__ V2Warp smem[V2_WPB];
     const uint32_t lane = lane_id(), wid = threadIdx.x >> 5;
     const uint64_t id = (uint64_t)blockIdx.x * V2_WPB + wid;  // 32 * chunk + lane stream
-    if (id >= n_lanes) return;                       // warp-uniform
+    if (id >= n_lanes || (skip && *skip)) return;  // warp-uniform
     V2Warp& S = smem[wid];
     const uint64_t cb = (id >> 5) * chunk_size;
     const uint64_t avail = (n_bytes > cb ? min((unsigned long long)(n_bytes - cb), (unsigned long long)chunk_size) : 0ull) / 8u;
