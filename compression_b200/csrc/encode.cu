@@ -461,6 +461,7 @@ inline uint64_t rlev2_lane_cap(uint64_t chunk_size) {
 //   128          2.39  1.44   1.06   1.14
 //   512          4.4   2.2    1.4    1.7
 //  1024          8.4   3.4    2.3    2.3
+// (8-byte values n = 64 1.66, 1.01, 0.68, 0.70)
 // and of runs of 8 equal values, which are a token each, n = 128 0.94, 0.39, 0.22,
 // 0.21, n = 1024 1.85, 0.61, 0.25, 0.22; RLE v2 n = 16 1.82, 1.07, 0.89, 0.78, n =
 // 1024 18.8, 7.4, 6.4, of runs n = 32 1.33, 0.89, 0.78, 0.58, n = 1024 1.75, 0.64,
@@ -469,8 +470,8 @@ inline uint64_t rlev2_lane_cap(uint64_t chunk_size) {
 // 14).  It and the launch that finds nothing to do take 6 to 8 us, which smaller
 // columns would feel (64 MiB in 128 KiB chunks 0.224 ms); there runs of 8 take
 // 0.50 ms by warps, 0.30 by threads.
-inline ThreadRule rlev1_by_thread(uint64_t lanes, uint64_t n) {
-    const bool all = n < 16 || (n < 32 && lanes >= 8192) || (n < 64 && lanes >= 32768) || (n < 128 && lanes >= 65536) ||
+inline ThreadRule rlev1_by_thread(uint64_t lanes, uint64_t n, uint32_t elem_bytes) {
+    const bool all = n < 16 || (n < 32 && lanes >= 8192) || (n < 64 && lanes >= 32768) || (n < 128 && lanes >= 262144 / elem_bytes) ||
                      (n < 256 && lanes >= 131072);
     return {all, !all && (lanes > 16384 || (n < 512 && lanes >= 16384)) ? SAMPLE : 0u};
 }
@@ -520,7 +521,7 @@ extern "C" gd_status_t gd_rlev1_encode_device(const uint8_t* d_in, uint64_t n_by
     const uint64_t nc = (n_bytes + chunk_size - 1) / chunk_size;
     auto go = [&](auto value) {
         using T = decltype(value);
-        const ThreadRule by = rlev1_by_thread(nc * 32u, chunk_size / 32u / sizeof(T));
+        const ThreadRule by = rlev1_by_thread(nc * 32u, chunk_size / 32u / sizeof(T), sizeof(T));
         uint64_t* runs = by.ends ? d_blk_off : nullptr;  // until the offsets are there
         if (runs)
             sample_runs_kernel<GD_CODEC_RLEV1, T>

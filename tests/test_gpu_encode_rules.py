@@ -22,7 +22,7 @@ def _column(rng, kind: str, n: int, dt) -> np.ndarray:
 @pytest.mark.parametrize("kind", ["runs", "values", "both"])
 @pytest.mark.parametrize("codec,elem,n,lanes", [
     ("rlev1", 4, 15, 64), ("rlev1", 4, 16, 8160), ("rlev1", 4, 16, 8192), ("rlev1", 4, 32, 32768), ("rlev1", 8, 63, 96),
-    ("rlev1", 8, 64, 16352), ("rlev1", 8, 64, 16384), ("rlev1", 4, 64, 65536), ("rlev1", 4, 512, 16416),
+    ("rlev1", 8, 64, 16352), ("rlev1", 8, 64, 16384), ("rlev1", 8, 64, 32768), ("rlev1", 4, 64, 65536), ("rlev1", 4, 512, 16416),
     ("rlev2", 8, 3, 64), ("rlev2", 8, 4, 8192), ("rlev2", 8, 16, 16384), ("rlev2", 8, 16, 32768), ("rlev2", 8, 32, 16384),
     ("rlev2", 8, 512, 16416)])
 def test_choice(cuda, codec, elem, n, lanes, kind):
