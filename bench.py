@@ -1188,6 +1188,10 @@ def run_reference(args, world):
                 "cpu_baseline": {"value": round(v, 3), "unit": "GB/s", "cores": threads, "kind": "port",
                                  "sample": f"host encoder on the whole column, {reps} passes"},
                 "e2e": {"value": round(v, 3), "unit": "GB/s", "h2d_bytes_per_step": 0, "d2h_bytes_per_step": 0}}
+    missing = [b for b in ("ref_brle", "ref_rlev2", "ref_lzss") if not (REF_BIN / b).exists()]
+    if missing:
+        return {"impl": "reference", "unavailable": f"{', '.join(missing)}: not built (oracle/ref/Makefile compiles them "
+                "from the reference's sources, which are not here)"}
     head = HEADLINE if w == "all" else w
     kern = []
     with tempfile.TemporaryDirectory() as td:

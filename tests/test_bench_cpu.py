@@ -6,6 +6,8 @@ import subprocess
 import sys
 from pathlib import Path
 
+import pytest
+
 ROOT = Path(__file__).resolve().parent.parent
 
 
@@ -16,6 +18,9 @@ def test_reference_arm_loads_no_product_library():
     line = json.loads(r.stdout.strip().splitlines()[-1])
     import bench
     assert line["impl"] == "reference"
+    if not (bench.REF_BIN / "ref_brle").exists():  # built from the reference's sources, where they are
+        assert "ref_brle" in line["unavailable"]
+        pytest.skip(line["unavailable"])
     assert line["metric"] == bench.HEADLINE_METRIC
     assert line["config"] == bench.run_config(bench.HEADLINE, 1)
     assert line["native_libs"] == ["oracle/liboracle.so"], line["native_libs"]
