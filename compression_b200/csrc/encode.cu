@@ -462,14 +462,15 @@ inline uint64_t rlev2_lane_cap(uint64_t chunk_size) {
 //   512          4.4   2.2    1.4    1.7
 //  1024          8.4   3.4    2.3    2.3
 // (8-byte values n = 64 1.66, 1.01, 0.68, 0.70)
-// and of runs of 8 equal values, which are a token each, n = 128 0.94, 0.39, 0.22,
-// 0.21, n = 1024 1.85, 0.61, 0.25, 0.22; RLE v2 n = 16 1.82, 1.07, 0.89, 0.78, n =
-// 1024 18.8, 7.4, 6.4, of runs n = 32 1.33, 0.89, 0.78, 0.58, n = 1024 1.75, 0.64,
-// 0.54.  So short lanes go by the sizes, and in columns of over 16,384 lanes
-// (n < 512: as many) a sample tells: an end of a run for every 32 values (RLE v2:
-// 14).  It and the launch that finds nothing to do take 6 to 8 us, which smaller
-// columns would feel (64 MiB in 128 KiB chunks 0.224 ms); there runs of 8 take
-// 0.50 ms by warps, 0.30 by threads.
+// RLE v2 n = 16 1.82, 1.07, 0.89, 0.78, n = 1024 18.8, 7.4, 6.4.  Of runs of 8
+// equal values, which are a token each, taken one by one: n = 128 0.94, 0.39, 0.22,
+// 0.21, n = 1024 1.85, 0.61, 0.25, 0.22; RLE v2 n = 32 1.33, 0.89, 0.78, 0.58, n =
+// 1024 1.75, 0.64, 0.54 (several at a time the warps take half as long).  So short
+// lanes go by the sizes, and in columns of over 16,384 lanes (n < 512: as many) a
+// sample tells: an end of a run for every 32 values (RLE v2: 14).  It and the
+// launch that finds nothing to do take 6 to 8 us, which smaller columns would feel
+// (64 MiB in 128 KiB chunks 0.222 ms; there runs of 8 take 0.23 ms by warps, 0.30
+// by threads).
 inline ThreadRule rlev1_by_thread(uint64_t lanes, uint64_t n, uint32_t elem_bytes) {
     const bool all = n < 16 || (n < 32 && lanes >= 8192) || (n < 64 && lanes >= 32768) || (n < 128 && lanes >= 262144 / elem_bytes) ||
                      (n < 256 && lanes >= 131072);

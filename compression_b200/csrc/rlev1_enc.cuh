@@ -8,8 +8,9 @@
 // up to the next run make groups of 127 at most.  So a warp takes a lane stream
 // token by token: the next run's place and length from two bit masks over the
 // values, a literal group's bytes from a prefix sum of its varints' lengths,
-// 32 values at a time.  A thread per lane stream, a value at a time, took
-// 0.63 ms for 64 MiB of the benchmark's column.
+// 32 values at a time; runs one after the other are taken together, a lane each
+// (64 MiB of runs of 8: 0.23 ms, one by one 0.49).  A thread per lane stream, a
+// value at a time, took 0.63 ms for 64 MiB of the benchmark's column.
 #pragma once
 #include "gd_common.cuh"
 
@@ -94,11 +95,11 @@ __global__ void __launch_bounds__(V1_WPB * 32) rlev1_encode_kernel(const uint8_t
         }
         __syncwarp();
         // bit k of E: values i + k .. i + k + 2 have one difference; of the lane's values only
-        uint32_t r = 127, z = 127;  // literals before the next run; equal differences from i on
+        uint32_t r = 127;  // literals before the next run
         const uint32_t valid = n - i > 2u ? n - i - 2u : 0u;
+        uint32_t E[4], P[4];
         {
             uint32_t e0 = S.eq[((i + 2u) >> 5) & 7u], s0 = S.small[((i + 1u) >> 5) & 7u];
-            uint32_t E[4], P[4];
 #pragma unroll
             for (uint32_t w = 0; w < 4; ++w) {
                 const uint32_t e1 = S.eq[(((i + 2u) >> 5) + w + 1u) & 7u];
@@ -110,13 +111,44 @@ __global__ void __launch_bounds__(V1_WPB * 32) rlev1_encode_kernel(const uint8_t
                 s0 = s1;
             }
 #pragma unroll
-            for (int w = 3; w >= 0; --w) {
+            for (int w = 3; w >= 0; --w)
                 if (P[w]) r = min(32u * w + __ffs(P[w]) - 1u, 127u);
-                if (~E[w]) z = min(32u * w + __ffs(~E[w]) - 1u, 127u);
-            }
         }
         uint8_t* out = S.out + on;
+        uint32_t z = 127;  // equal differences from i on
         if (r == 0) {
+#pragma unroll
+            for (int w = 3; w >= 0; --w)
+                if (~E[w]) z = min(32u * w + __ffs(~E[w]) - 1u, 127u);
+        }
+        if (r == 0 && z < 30u && (P[0] >> (z + 2u) & 1u)) {
+            // runs one after the other, as many as the masks show the ends
+            // of (their bit 126 is the last that is known): a lane each
+            const uint64_t e0 = (uint64_t)E[1] << 32 | E[0], e1 = (uint64_t)E[3] << 32 | E[2];
+            const uint64_t p0 = (uint64_t)P[1] << 32 | P[0], p1 = (uint64_t)P[3] << 32 | P[2];
+            uint32_t at = 0, k = 0, start = 0, L = 0;
+            while (k < 32u && at < 126u && ((at < 64u ? p0 >> at : p1 >> (at - 64u)) & 1u)) {
+                const uint64_t x = at == 0u ? e0 : at < 64u ? e0 >> at | e1 << (64u - at) : e1 >> (at - 64u);
+                const uint32_t ones = (uint32_t)__ffsll((long long)~x) - 1u;  // all ones: none
+                if (ones >= 64u || at + ones > 126u) break;
+                if (lane == k) {
+                    start = at;
+                    L = 2u + ones;
+                }
+                at += 2u + ones;
+                ++k;
+            }
+            const T v = S.ring[(i + start) & 255u], d = S.ring[(i + start + 1u) & 255u] - v;
+            const uint32_t nb = v1_varint_len(v), size = lane < k ? 2u + nb : 0u, inc = warp_incl_scan(size);
+            if (lane < k) {
+                uint8_t* o = out + inc - size;
+                o[0] = (uint8_t)(L - 3u);
+                o[1] = (uint8_t)d;
+                v1_put_varint(v, nb, o + 2);
+            }
+            on += __shfl_sync(GD_FULL_MASK, inc, 31);
+            i += at;
+        } else if (r == 0) {
             const uint32_t L = 2u + z;
             const T v = S.ring[i & 255u], d = S.ring[(i + 1u) & 255u] - v;
             const uint32_t nb = v1_varint_len(v);

@@ -287,6 +287,7 @@ inline T __ldg(const T* p) { return *p; }
 
 inline int __popc(uint32_t x) { return std::popcount(x); }
 inline int __ffs(uint32_t x) { return x ? std::countr_zero(x) + 1 : 0; }
+inline int __ffsll(long long x) { return x ? std::countr_zero((uint64_t)x) + 1 : 0; }
 inline int __clz(uint32_t x) { return std::countl_zero(x); }
 inline int __clzll(long long x) { return std::countl_zero((uint64_t)x); }
 inline uint32_t __brev(uint32_t x) {

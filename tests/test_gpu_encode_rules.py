@@ -39,3 +39,31 @@ def test_choice(cuda, codec, elem, n, lanes, kind):
     for k in want.meta:
         assert np.array_equal(want.meta[k], got.meta[k]), k
     assert np.array_equal(want.data, got.data)
+
+
+@pytest.mark.parametrize("codec,elem", [("rlev1", 4), ("rlev1", 8), ("rlev2", 8)])
+def test_short_runs_in_a_row(cuda, codec, elem):
+    """Runs that a warp takes together: of 3 to 70 values, values of every
+    width, up to the ends of the window and of the lane, literals between."""
+    rng = np.random.default_rng(elem)
+    n, dt = 700, np.int32 if elem == 4 else np.int64
+    lanes = []
+    for q in range(32):
+        x = []
+        while len(x) < n:
+            k = int(rng.choice([3, 4, 5, 8, 9, 10, 11, 12, 30, 31, 32, 63, 64, 65, 70][:15 - q % 8]))
+            base = int(rng.integers(-1 << int(rng.integers(1, 8 * elem - 1)), 1 << int(rng.integers(1, 8 * elem - 1))))
+            x += [base + i * (int(rng.integers(-5, 6)) if codec == "rlev1" and q % 3 == 0 else 0) for i in range(k)]
+            if q % 4 == 1 and rng.random() < 0.1:
+                x += rng.integers(0, 1000, int(rng.integers(1, 40))).tolist()
+        lanes.append(np.array(x[:n], np.int64).astype(dt))
+    raw = np.concatenate(lanes)  # slices as long as the lanes: lane after lane
+    if codec == "rlev1":
+        want = cc.rlev1_encode(raw, raw.nbytes, n * elem, elem)
+        got = cc.encode_gpu("rlev1", raw, raw.nbytes, comp_col_len=n * elem, elem_bytes=elem)
+    else:
+        want = cc.rlev2_encode(raw, raw.nbytes, n)
+        got = cc.encode_gpu("rlev2", raw, raw.nbytes, read_unit=n)
+    for k in want.meta:
+        assert np.array_equal(want.meta[k], got.meta[k]), k
+    assert np.array_equal(want.data, got.data)
