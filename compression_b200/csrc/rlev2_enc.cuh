@@ -7,6 +7,8 @@
 // written as a delta run (`stale` below).  So a warp takes a lane stream run by
 // run: the run's end from a bit mask of equal neighbours, its encoding from
 // warp reductions over at most 128 values (four a lane), its bytes one a lane.
+// Short runs of equal values one after the other are taken together, a lane each
+// (64 MiB: the benchmark's column 0.298 -> 0.278 ms, runs of 8 0.28 -> 0.15).
 // A thread per lane stream, each with 6 KB of run buffers in local memory and
 // branching on its own run, took 5.5 ms for 64 MiB of the benchmark's column.
 //
@@ -368,7 +370,35 @@ __global__ void __launch_bounds__(V2_WPB * 32) rlev2_encode_kernel(const uint8_t
             if (tri) j = 32u * w + __ffs(tri) - 1u;
         }
         uint8_t* out = S.out + on;
-        if (e >= 3) {
+        if (e >= 3 && e <= 10 && (E[0] >> e & 3u) == 3u) {
+            // short runs one after the other, as many as the mask shows the
+            // ends of (its bit 126 is the last that is known): a lane each
+            const uint64_t lo = (uint64_t)E[1] << 32 | E[0], hi = (uint64_t)E[3] << 32 | E[2];
+            uint32_t at = 0, k = 0, start = 0, m = 0;
+            while (k < 32u && at < 126u) {
+                const uint64_t x = at == 0u ? lo : at < 64u ? lo >> at | hi << (64u - at) : hi >> (at - 64u);
+                const uint32_t ones = (uint32_t)__ffsll((long long)~x) - 1u;  // all ones: none
+                if (ones - 2u > 7u || at + ones > 126u) break;
+                if (lane == k) {
+                    start = at;
+                    m = ones + 1u;
+                }
+                at += ones + 1u;
+                ++k;
+            }
+            const int64_t v = S.ring[(i + start) & 255u];
+            const uint32_t nb = v < 0 ? 8u : (enc::w_closest(v2_bits((uint64_t)v)) + 7u) / 8u;
+            const uint32_t size = lane < k ? 1u + nb : 0u, inc = warp_incl_scan(size);
+            if (lane < k) {
+                uint8_t* o = out + inc - size;
+                o[0] = (uint8_t)(((nb - 1u) << 3) | (m - 3u));
+#pragma unroll
+                for (uint32_t b = 0; b < 8; ++b)
+                    if (b < nb) o[1 + b] = (uint8_t)((uint64_t)v >> (8u * (nb - 1u - b)));
+            }
+            on += __shfl_sync(GD_FULL_MASK, inc, 31);
+            i += at;
+        } else if (e >= 3) {
             const int64_t v = S.ring[i & 255u];
             if (e <= 10) {
                 const uint32_t nb = v < 0 ? 8u : (enc::w_closest(v2_bits((uint64_t)v)) + 7u) / 8u;
